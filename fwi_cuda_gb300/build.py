@@ -33,6 +33,7 @@ UNITS = [
     ("psv_kernels_f32.cu", []),
     ("psv_kernels_f64.cu", []),
     ("psv_tiled.cu", []),
+    ("psv_loop.cu", []),
     ("psv_vec.cu", []),
     ("psv_fused.cu", []),
     ("psv_march.cu", []),

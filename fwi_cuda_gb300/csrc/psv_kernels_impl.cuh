@@ -319,12 +319,11 @@ struct TileSR {
     int k0, k1, r0, r1;
 };
 template <typename T>
-__device__ __forceinline__ TileSR tile_srcrec(const StepParams<T> &p, const SrcRecParams<T> &q,
-                                              int tile, int bz)
+__device__ __forceinline__ TileSR tile_srcrec(const SrcRecParams<T> &q, int shot0, int tile, int bz)
 {
     TileSR s{0, 0, 0, 0};
     if (q.src_kind == 0) {
-        const int *off = q.t_src_off + (long long)(p.ctl[0] + bz) * (q.ntiles + 1);
+        const int *off = q.t_src_off + (long long)(shot0 + bz) * (q.ntiles + 1);
         s.k0 = off[tile];
         s.k1 = off[tile + 1];
     } else if (q.src_kind == 1) {
@@ -336,6 +335,13 @@ __device__ __forceinline__ TileSR tile_srcrec(const StepParams<T> &p, const SrcR
         s.r1 = q.t_rec_off[tile + 1];
     }
     return s;
+}
+
+template <typename T>
+__device__ __forceinline__ TileSR tile_srcrec(const StepParams<T> &p, const SrcRecParams<T> &q,
+                                              int tile, int bz)
+{
+    return tile_srcrec(q, p.ctl[0], tile, bz);
 }
 
 // vsrc2 + urec2 (src/cpu/n_kernel_lib_PSV.cpp:487-576) for the sources and

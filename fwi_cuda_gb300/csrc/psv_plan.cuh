@@ -35,12 +35,43 @@ struct TileMaps {
     CUtensorMap coef;  // coefficient planes, box 64 x 4 rpt
 };
 // 3-D tensor map (column, row, plane) over nplanes planes of nz x nx floats
-// (row pitch `pitch`, plane stride `plane` elements), box bx x by x 1, zero
+// (row pitch `pitch`, plane stride `plane` elements), box bx x by x bp, zero
 // fill outside (psv_tiled.cu).
 int encode3(CUtensorMap *map, const float *base, int nx, int nz, int pitch, long long plane,
-            int nplanes, int bx, int by);
+            int nplanes, int bx, int by, int bp = 1);
 int encode_tile_maps(TileMaps *m, const float *fld, int nfplanes, const float *coef, int nx, int nz,
                      int pitch, long long plane, int ns, int rpt);
+// Many steps of the TMA family in one launch (FP32, psv_loop.cu): tiles of 64
+// columns x tz rows (8 or 16).  Maps: boxes of 2 or 3 adjacent planes.
+struct LoopMaps {
+    CUtensorMap halo2, halo3;      // v, sigma with the stencil halo
+    CUtensorMap own1, own2, own3;  // a tile of We, of v or u, of sigma
+    CUtensorMap hist5, grad3;      // a tile of a snapshot, of a shot's gradients (unit spacing only)
+};
+// Steps it0, it0 + dit, ... of a launch.  snap: steps divisible by sdt store
+// or image snapshot slot (it / sdt - base) % ring.  far: the wavefields do not
+// fit in L2; images: snapshot slots per shot that hist5 covers (0: no map).
+// keep: see keep_sum in psv_loop.cu.  sync: device words, the item counter and, from LOOP_SYNC_HEAD on, the tiles'
+// progress words.
+struct LoopRun {
+    int nsteps, it0, dit;
+    int sdt, base, ring, snap;
+    int far, images;
+    const int *keep;  // per tile: sums keep what they round off (forward modes), or null
+    int *sync;
+};
+constexpr int LOOP_SYNC_HEAD = 32;
+cudaError_t launch_loop_kept(int op, float *fld, long long shot_stride, long long plane, int pitch, int nz, int nx,
+                             int tz, const int *tiles, int ntiles, float *packed, long long cstride, int nbatch,
+                             cudaStream_t st);
+bool loop_supported(int tz, int st, int sb, int sl, int sr, int nz1);
+size_t loop_sync_bytes(int nz, int nx, int nbatch);
+int loop_max_steps(int nz, int nx, int nbatch);
+int encode_loop_maps(LoopMaps *m, const float *fld, int nfplanes, int nx, int nz, int pitch,
+                     long long plane, int ns, int tz, const float *hist, int nhplanes, const float *gshot,
+                     int ngplanes, int snx_pitch, int snz);
+cudaError_t launch_loop(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopMaps &m,
+                        const LoopRun &run, int ns, int mode, int tz, int nbatch, cudaStream_t st);
 // Four-columns-per-thread kernels (FP32, psv_vec.cu): blocks of 32 x by
 // threads over 128 columns x by * rpt rows, rpt in {1, 2, 4}.
 cudaError_t launch_stress_v4(const StepParams<float> &p, int ns, int rpt, int by, int nbatch,

@@ -54,6 +54,7 @@ public:
     psv_options opt;
     int B = 1, nbatch = 1;
     int pitch = 0, mx_pitch = 0, snx_pitch = 0, nzs = 0, nxs = 0;
+    int snx_off = 0;  // first column of the snapshot window within its stored rows
     long long plane = 0, shot_stride = 0, mz_shot = 0, mx_shot = 0, hist_shot = 0, gshot_shot = 0;
     long long ntr = 0;  // nt * nrec
     size_t total = 0;
@@ -67,6 +68,11 @@ public:
     int rpt = 1;                                     // rows per thread (< 0: shuffle variant)
     int fam = PSV_KERNELS_DIRECT;                    // kernel family of the time step
     TileMaps tmap{}, tmap2{};                        // tensor maps of fld / fld2 (TMA family)
+    LoopMaps lmap{}, lmap2{};                        // ... and of its many-step launches
+    DevMem lsync;                                    // their item counter and progress words
+    DevMem lkeep, lkept;                             // per tile: keeps its sums' roundings; those tiles
+    int nkept = 0;
+    long long ck_kept = 0;  // elements of a checkpointed state that hold them
     MarchMaps mmap{}, mmap2{};                       // tensor maps of fld / fld2 (MARCH family)
     int *h_err = nullptr;                            // pinned copy of the device error word
     std::vector<int> h_f_off;                        // host copy of the per-shot source lists
@@ -212,12 +218,23 @@ public:
             return fail(PSV_ERR_UNSUPPORTED, "grid too large: one shot's field planes exceed "
                                              "2^31 - 1 elements (nz x padded nx x " +
                                                  std::to_string(nfield()) + " planes)");
+        if (sizeof(T) == 4 && g.pml_x) {
+            // x strips that start and end on multiples of four columns: the
+            // added columns' profiles are the identity, and 128-bit accesses
+            // then fall inside a strip or outside it
+            sv.px0 = (sv.px0 + 3) & ~3;
+            if (sv.px1 < nx) sv.px1 &= ~3;
+            if (sv.px0 >= sv.px1) sv.px0 = sv.px1 = nx;  // all strip
+        }
         nzs = g.pml_z ? sv.pz0 + (nz - sv.pz1) : 0;
         nxs = g.pml_x ? sv.px0 + (nx - sv.px1) : 0;
         mx_pitch = nxs ? round_up(nxs, al) : 0;
         mz_shot = (long long)(sizeof(T) == 4 ? NMZ_PP : NMZ) * nzs * pitch;
         mx_shot = (long long)(sizeof(T) == 4 ? NMX_PP : NMX) * nz * mx_pitch;
-        snx_pitch = round_up(sv.snx, al);
+        // Stored rows start so that a window column has its grid column's
+        // alignment (128-bit stores and loads of whole quads).
+        snx_off = sizeof(T) == 4 && g.snap_dx == 1 ? g.snap_x1 & 3 : 0;
+        snx_pitch = round_up(sv.snx + snx_off, al);
         const long long snap_plane = (long long)sv.snz * snx_pitch;
         hist_shot = (long long)sv.snt * NHIST * snap_plane;
         gshot_shot = 3 * snap_plane;
@@ -247,6 +264,9 @@ public:
             while (b > 1 && shared + b * (per_shot + extra) > budget) b--;
             return shared + b * (per_shot + extra) <= budget ? b : 0;
         };
+        if (sizeof(T) == 4)  // a state also holds the kept roundings of the looped tiles
+            ck_kept = 5 * 64 * (long long)std::max(8 * kept_tiles(8).size(), 16 * kept_tiles(16).size());
+        ck_state += ck_kept;
         const int b_full = fit(per_hist);
         int b_ck = binomial ? 0 : fit(per_ck(nseg));
         nck = nseg;
@@ -290,6 +310,16 @@ public:
         }
         if (ckpt) hist_shot = (long long)nslots * NHIST * snap_plane;
         nbatch = (nshot + B - 1) / B;
+        // The shape of a plan nobody autotunes (modelling).  From 500 000
+        // points in a batch the looped TMA tiles beat the direct kernels:
+        // 12.7 against 14.1 us a step at 0.54 M points (301 x 601, 3 shots,
+        // order 4), 16.5 against 25.9 at 1.4 M, 21 against 40 at 2.0 M
+        // (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
+        if (sizeof(T) == 4 && opt.kernel_family == 0 && opt.rows_per_thread == 0 && opt.block_y <= 0 &&
+            (double)nz * nx * B >= 500e3 && loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
+            fam = PSV_KERNELS_TMA;
+            rpt = 4;
+        }
 
         PSV_CU(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         for (auto &e : ev) PSV_CU(cudaEventCreate(&e));
@@ -313,13 +343,14 @@ public:
         PSV_TRY(memx.alloc((size_t)B * mx_shot * sizeof(T), total));
         PSV_TRY(gshot.alloc((size_t)B * gshot_shot * sizeof(T), total));
         PSV_TRY(coef.alloc((size_t)7 * plane * sizeof(T), total));
-        const int nmax = std::max(nz, nx);
+        const int nmax = profile_len();
         PSV_TRY(prof.alloc((size_t)12 * nmax * sizeof(T), total));
         PSV_TRY(fsb.alloc((size_t)(2 * nx + 2 * nz) * sizeof(T), total));
         PSV_TRY(model.alloc((size_t)12 * nz * nx * 8, total));
         PSV_TRY(traces.alloc((size_t)6 * nshot * ntr * 8 + 8, total));
         PSV_TRY(red.alloc(((size_t)256 * std::max(3, nshot) + nshot + 3 + B + 2) * 8, total));
         PSV_TRY(taperb.alloc((size_t)(nx + nz) * 8, total));
+        if (sizeof(T) == 4) PSV_TRY(lsync.alloc(loop_sync_bytes(nz, nx, B), total));
         PSV_TRY(ctl.alloc(4 * sizeof(int), total));
         PSV_TRY(ctl2.alloc(2 * MAXCH * sizeof(int), total));
         PSV_CU(cudaMemsetAsync(ctl2.p, 0, 2 * MAXCH * sizeof(int), st));
@@ -345,6 +376,8 @@ public:
         return PSV_OK;
     }
 
+    // Length of a CPML profile on the device (128-byte rows).
+    int profile_len() const { return round_up(std::max(sv.g.nz, sv.g.nx), 32); }
     static int tma_rpt(int r) { return (r == 2 || r == 4 || r == 8) ? r : 4; }
     static int fused_tz(int r) { return (r == 16 || r == 32) ? r : 32; }
     bool fused_ok(int tz) const
@@ -364,6 +397,82 @@ public:
     }
     // One launch per step, v and sigma ping-ponged (FUSED tiles or MARCH strips).
     bool fused() const { return fam == PSV_KERNELS_FUSED || fam == PSV_KERNELS_MARCH; }
+    // Many steps per launch (psv_loop.cu): the TMA family, except with bottom or
+    // side surfaces or mirrored rows beyond the first tile, whose mirror writes
+    // cross tiles (those step through psv_tiled.cu).
+    bool looped() const
+    {
+        return sizeof(T) == 4 && fam == PSV_KERNELS_TMA &&
+               loop_supported(4 * rpt, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1);
+    }
+    // Snapshot slots per shot that a tensor map of the history covers (0: none,
+    // not allocated or the window is subsampled).
+    int image_slots() const
+    {
+        return hist.p && sv.g.snap_dx == 1 && sv.g.snap_dz == 1 ? (ckpt ? nslots : sv.snt) : 0;
+    }
+    // Tiles of 64 columns x tz rows within eight cells of a source or receiver:
+    // their sums keep what they round off on forward passes (keep_sum).
+    std::vector<int> kept_tiles(int tz) const
+    {
+        const int ntx = (sv.g.nx + 63) / 64, ntz = (sv.g.nz + tz - 1) / tz;
+        std::vector<char> on((size_t)ntx * ntz, 0);
+        auto mark = [&](int z, int x) {
+            for (int b = std::max(z - 8, 0) / tz; b <= std::min(z + 8, sv.g.nz - 1) / tz; b++)
+                for (int c = std::max(x - 8, 0) / 64; c <= std::min(x + 8, sv.g.nx - 1) / 64; c++)
+                    on[(size_t)b * ntx + c] = 1;
+        };
+        for (int i = 0; i < sv.s.nsrc; i++) mark(sv.z_src[i], sv.x_src[i]);
+        for (int i = 0; i < sv.s.nrec; i++) mark(sv.z_rec[i], sv.x_rec[i]);
+        std::vector<int> t;
+        for (size_t k = 0; k < on.size(); k++)
+            if (on[k]) t.push_back((int)k);
+        return t;
+    }
+    int build_kept()
+    {
+        nkept = 0;
+        if (!looped()) return PSV_OK;
+        const int tz = 4 * rpt;
+        const std::vector<int> t = kept_tiles(tz);
+        std::vector<int> on((size_t)((sv.g.nx + 63) / 64) * ((sv.g.nz + tz - 1) / tz), 0);
+        for (int k : t) on[(size_t)k] = 1;
+        PSV_TRY(put(lkeep, on));
+        PSV_TRY(put(lkept, t));
+        nkept = (int)t.size();
+        return PSV_OK;
+    }
+    // Zero (op 0) the kept roundings of state s, or copy them to (1) / from (2)
+    // the end of a checkpointed state.
+    cudaError_t kept(int op, const StepParams<T> &s, T *state)
+    {
+        if constexpr (sizeof(T) == 4)
+            if (looped())
+                return launch_loop_kept(op, s.fld + (long long)s.pp_planes * plane, s.shot_stride, plane, pitch,
+                                        sv.g.nz, sv.g.nx, 4 * rpt, lkept.as<int>(), nkept,
+                                        state ? state + ck_state - ck_kept : nullptr, ck_state, B, st);
+        return cudaSuccess;
+    }
+    // n steps it0, it0 + dit, ... of a looped plan; snapshot steps use slot
+    // (it / snap_dt - base) % ring where `snap`.
+    int loop_steps(const StepParams<T> &s, const SrcRecParams<T> &q, int mode, bool second, int it0,
+                   int dit, int n, bool snap, int base, int ring, long long &nk)
+    {
+        if constexpr (sizeof(T) == 4) {
+            const int most = loop_max_steps(sv.g.nz, sv.g.nx, B);
+            // the fields a step touches, against what L2 holds beside the rest
+            const double state = (mode == MODE_ADJ ? 8.0 : mode == MODE_FWD ? 6.0 : 5.0) * plane * B * sizeof(T);
+            const int far = state > 90e6;
+            for (int j = 0; j < n; j += most) {
+                const LoopRun run{std::min(most, n - j), it0 + j * dit, dit, sv.g.snap_dt, base,
+                                  std::max(ring, 1), snap, far, mode == MODE_ADJ ? image_slots() : 0,
+                                  nkept ? lkeep.as<int>() : nullptr, lsync.as<int>()};
+                PSV_CU(launch_loop(s, q, second ? lmap2 : lmap, run, sv.ns, mode, 4 * rpt, B, st));
+                nk++;
+            }
+        }
+        return PSV_OK;
+    }
     // Copy of v and sigma a step reads: step k of a pass reads copy k & 1
     // (the fused family ping-pongs; the others update in place, copy 0).
     int par(int k) const { return fused() ? (k & 1) : 0; }
@@ -386,6 +495,13 @@ public:
             if (fam != PSV_KERNELS_TMA) return PSV_OK;
             PSV_TRY(encode_tile_maps(&tmap, fld.as<float>(), (int)(B * nfield()), coef.as<float>(),
                                      g.nx, g.nz, pitch, plane, sv.ns, rpt));
+            if (looped())
+                PSV_TRY(encode_loop_maps(&lmap, fld.as<float>(), (int)(B * nfield()), g.nx, g.nz, pitch,
+                                         plane, sv.ns, 4 * rpt, image_slots() ? hist.as<float>() : nullptr,
+                                         B * image_slots() * NHIST, gshot.as<float>(), 3 * B, snx_pitch, sv.snz));
+            if (looped() && fld2.p)
+                PSV_TRY(encode_loop_maps(&lmap2, fld2.as<float>(), B * nwork(), g.nx, g.nz, pitch, plane,
+                                         sv.ns, 4 * rpt, nullptr, 0, nullptr, 0, 0, 0));
             if (fld2.p)
                 PSV_TRY(encode_tile_maps(&tmap2, fld2.as<float>(), B * nwork(), coef.as<float>(), g.nx,
                                          g.nz, pitch, plane, sv.ns, rpt));
@@ -519,7 +635,7 @@ public:
 
     int upload_profiles()
     {
-        const int nz = sv.g.nz, nx = sv.g.nx, nmax = std::max(nz, nx);
+        const int nz = sv.g.nz, nx = sv.g.nx, nmax = profile_len();
         std::vector<T> h((size_t)12 * nmax, T(0));
         for (int a = 0; a < 12; a++) {
             const bool zaxis = a < 6;
@@ -632,7 +748,7 @@ public:
         PSV_TRY(put(t_src_k, sk));
         PSV_TRY(put(t_rec_off, roff));
         PSV_TRY(put(t_rec_r, rr));
-        return PSV_OK;
+        return build_kept();
     }
 
     int snap_cell(int iz, int ix) const
@@ -687,7 +803,7 @@ public:
     void fill_params()
     {
         const psv_grid &g = sv.g;
-        const int nz = g.nz, nx = g.nx, nmax = std::max(nz, nx);
+        const int nz = g.nz, nx = g.nx, nmax = profile_len();
         StepParams<T> &p = sp;
         p = StepParams<T>{};
         p.nz = nz; p.nx = nx; p.pitch = pitch;
@@ -726,8 +842,8 @@ public:
         p.snap_plane = (long long)sv.snz * snx_pitch;
         p.hist_slot_stride = NHIST * p.snap_plane;
         p.hist_shot_stride = hist_shot;
-        p.hist = hist.as<T>();
-        p.gshot = gshot.as<T>();
+        p.hist = hist.as<T>() + snx_off;
+        p.gshot = gshot.as<T>() + snx_off;
         p.gshot_shot_stride = gshot_shot;
         p.ctl = ctl.as<int>();
         p.err = ctl.as<int>() + 2;
@@ -772,7 +888,7 @@ public:
     {
         if (hist.p || hist_shot == 0) return PSV_OK;
         PSV_TRY(hist.alloc((size_t)B * hist_shot * sizeof(T), total));
-        sp.hist = hist.as<T>();
+        sp.hist = hist.as<T>() + snx_off;
         if (ckpt) {
             PSV_TRY(ck.alloc((size_t)nck * B * ck_state * sizeof(T), total));
             PSV_TRY(fld2.alloc((size_t)B * nwork() * plane * sizeof(T), total));
@@ -784,7 +900,7 @@ public:
             sp2.memz = memz2.as<T>();
             sp2.memx = memx2.as<T>();
         }
-        sp2.hist = hist.as<T>();
+        sp2.hist = hist.as<T>() + snx_off;
         PSV_TRY(encode_maps());
         drop_graphs();
         return PSV_OK;
@@ -819,6 +935,7 @@ public:
             if (save) PSV_CU(cudaMemcpy2DAsync(cx, cp, mx, xw, xw, B, cudaMemcpyDeviceToDevice, st));
             else PSV_CU(cudaMemcpy2DAsync(mx, xw, cx, cp, xw, B, cudaMemcpyDeviceToDevice, st));
         }
+        PSV_CU(kept(save ? 1 : 2, main ? sp : sp2, c));
         return PSV_OK;
     }
 
@@ -837,6 +954,13 @@ public:
                 PSV_TRY(chained_steps(
                     sp2, qr, MODE_FWD_NOWE, e - a, [&](int j) { return a + j; },
                     [](int) { return -1; }, true, nk));
+            } else if (x.op == CK_ADVANCE && looped()) {
+                PSV_TRY(loop_steps(sp2, qr, MODE_FWD_NOWE, true, a, 1, e - a, false, 0, 1, nk));
+            } else if (x.op == CK_REVERSE && looped()) {
+                const int base = (a + sdt - 1) / sdt, last = (e - 1) / sdt * sdt;
+                PSV_TRY(loop_steps(sp2, qr, MODE_FWD_NOWE, true, a, 1, std::max(last - a + 1, 0), true,
+                                   base, nslots, nk));
+                PSV_TRY(loop_steps(sp, qa, MODE_ADJ, false, e - 1, -1, e - a, true, base, nslots, nk));
             } else if (x.op == CK_ADVANCE) {
                 for (int it = a; it < e; it++)
                     PSV_CU(step(sp2, qr, MODE_FWD_NOWE, it, -1, true, par(it)));
@@ -905,6 +1029,7 @@ public:
         }
         PSV_CU(launch_zero_planes<T>(memz.as<T>(), mz_shot, 0, mz_shot, B, st));
         PSV_CU(launch_zero_planes<T>(memx.as<T>(), mx_shot, 0, mx_shot, B, st));
+        if (mode != MODE_ADJ) PSV_CU(kept(0, sp, nullptr));
         long long nk = (mode == MODE_ADJ ? 5 : mode == MODE_FWD ? 4 : 3);
         if (ckpt && kind == PASS_FWD_STORE && chained()) {
             // one segment at a time: its state saved, then its steps on the chains
@@ -914,6 +1039,12 @@ public:
                 PSV_TRY(chained_steps(
                     sp, qf, mode, std::min(K, nt - a), [&](int j) { return a + j; },
                     [](int) { return -1; }, false, nk));
+            }
+        } else if (ckpt && kind == PASS_FWD_STORE && looped()) {
+            for (int a = 0; a < nt; a += K) {
+                if (fwd_slot[(size_t)(a / K)] >= 0)
+                    PSV_TRY(ck_copy(fwd_slot[(size_t)(a / K)], CK_SAVE_MAIN, 0));
+                PSV_TRY(loop_steps(sp, qf, mode, false, a, 1, std::min(K, nt - a), false, 0, 1, nk));
             }
         } else if (ckpt && kind == PASS_FWD_STORE) {
             // forward saving the schedule's states at the starts of their segments
@@ -925,6 +1056,9 @@ public:
             nk += lps() * nt;
         } else if (ckpt && kind == PASS_ADJ_RES) {
             PSV_TRY(run_schedule(nk));
+        } else if (looped()) {
+            PSV_TRY(loop_steps(sp, q, mode, false, adj ? nt - 1 : 0, adj ? -1 : 1, nt, store || adj, 0,
+                               sv.snt, nk));
         } else if (chained()) {
             PSV_TRY(enqueue_chained(q, mode, adj, store, nk));
         } else {
@@ -1176,7 +1310,7 @@ public:
         }
         const size_t bytes = (size_t)n * gshot_shot * sizeof(T);
         PSV_CU(cudaMemcpyAsync(gtmp.p, gshot.p, bytes, cudaMemcpyDeviceToDevice, st));
-        PSV_CU(launch_gauss_filter<T>(gtmp.as<T>(), gshot.as<T>(), sp.snap_plane, snx_pitch, sv.snz,
+        PSV_CU(launch_gauss_filter<T>(gtmp.as<T>() + snx_off, sp.gshot, sp.snap_plane, snx_pitch, sv.snz,
                                       sv.snx, 3 * n, gfilt.as<double>(), hfs, st));
         return PSV_OK;
     }
@@ -1209,7 +1343,7 @@ public:
         s.z1 = g.snap_z1; s.z2 = g.snap_z2; s.x1 = g.snap_x1; s.x2 = g.snap_x2;
         s.sdz = g.snap_dz; s.sdx = g.snap_dx; s.snx_pitch = snx_pitch;
         s.snap_plane = sp.snap_plane;
-        s.gshot = gshot.as<T>(); s.gshot_shot_stride = gshot_shot;
+        s.gshot = sp.gshot; s.gshot_shot_stride = gshot_shot;
         s.fld = fld.as<T>(); s.plane = plane; s.shot_stride = shot_stride;
         s.wmax = wmax();
         s.fscale = fscale(); s.ascale = ascale(); s.s0 = last_batch_s0;
@@ -1359,7 +1493,7 @@ public:
                 for (int jz = 0; jz < sv.snz; jz++)
                     for (int jx = 0; jx < sv.snx; jx++)
                         o[k][(size_t)jz * sv.snx + jx] =
-                            (double)h[k * sp.snap_plane + (size_t)jz * snx_pitch + jx] * gun[k];
+                            (double)h[k * sp.snap_plane + (size_t)jz * snx_pitch + snx_off + jx] * gun[k];
         double *w[2] = {We, WeA};
         const int wp[2] = {F_WE, F_WEA};
         const double wun[2] = {1.0 / (sf * sf), 1.0 / (sa * sa)};
@@ -1509,7 +1643,9 @@ public:
 
     int autotune(int nsteps, int *out_fam, int *out_rpt, int *out_by) override
     {
-        const TuneKey key{sv.g.nz, sv.g.nx, sv.ns, B, (int)sizeof(T), opt.kernel_family};
+        // (plans the loops cannot serve choose among other kernels)
+        const TuneKey key{sv.g.nz, sv.g.nx, sv.ns, B, (int)sizeof(T),
+                          opt.kernel_family + (loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) ? 0 : 16)};
         auto report = [&] {
             if (out_fam) *out_fam = fam;
             if (out_rpt) *out_rpt = rpt;
@@ -1537,7 +1673,7 @@ public:
             }
         }
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_TMA))
-            for (int r : {2, 4, 8}) cand.emplace_back(PSV_KERNELS_TMA, r, 4);
+            for (int r : {2, 4}) cand.emplace_back(PSV_KERNELS_TMA, r, 4);
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_VEC4))
             for (int r : {1, 2, 4})
                 for (int by : {2, 4, 8}) cand.emplace_back(PSV_KERNELS_VEC4, r, by);
@@ -1548,24 +1684,32 @@ public:
             for (int rows : {32, 64, 128})
                 for (int w : {2, 4})
                     if (march_ok(rows, w)) cand.emplace_back(PSV_KERNELS_MARCH, rows, w);
-        // 1) every candidate, launch by launch with CUDA events
+        // 1) every candidate, launch by launch with CUDA events; the looped
+        // ones have no launches of one step and go to 2) as they are
         std::vector<std::pair<double, std::tuple<int, int, int>>> timed;
+        std::vector<std::tuple<int, int, int>> loops;
         for (auto &c : cand) {
             PSV_TRY(set_shape(std::get<0>(c), std::get<1>(c), std::get<2>(c)));
+            if (looped()) {
+                loops.emplace_back(fam, rpt, (int)blk.y);
+                continue;
+            }
             double ms[6];
             PSV_TRY(profile(nsteps, ms));
             timed.emplace_back(ms[0] + ms[1] + ms[3] + ms[4], std::make_tuple(fam, rpt, (int)blk.y));
         }
         std::sort(timed.begin(), timed.end(),
                   [](const auto &a, const auto &b) { return a.first < b.first; });
-        // 2) the three fastest again as graph-replayed bursts of forward +
+        if (timed.size() > 3) timed.resize(3);
+        for (auto &c : loops) timed.emplace_back(0.0, c);
+        // 2) the three fastest and the loops as graph-replayed bursts of forward +
         // adjoint steps, the way the passes run, with 1, 2 and 4 chains for
         // the direct family (chaining can reorder them)
         std::tuple<int, int, int> pick = timed.empty() ? std::make_tuple(fam, rpt, (int)blk.y)
                                                        : timed.front().second;
         int ck = chains;
         double tb = 1e30;
-        for (size_t i = 0; i < std::min<size_t>(3, timed.size()); i++) {
+        for (size_t i = 0; i < timed.size(); i++) {
             const auto &sh = timed[i].second;
             PSV_TRY(set_shape(std::get<0>(sh), std::get<1>(sh), std::get<2>(sh)));
             const bool chainable = opt.chains == 0 && fam == PSV_KERNELS_DIRECT && B >= 2;
@@ -1845,6 +1989,9 @@ public:
             const int mode = adj ? MODE_ADJ : MODE_FWD;
             if (chained()) {
                 PSV_TRY(enqueue_chained(q, mode, adj, true, nk, nsteps));
+            } else if (looped()) {
+                PSV_TRY(loop_steps(sp, q, mode, false, adj ? sv.g.nt - 1 : 0, adj ? -1 : 1, nsteps, true, 0,
+                                   ckpt ? nslots : sv.snt, nk));
             } else {
                 const int nt = sv.g.nt, sdt = sv.g.snap_dt;
                 for (int j = 0; j < nsteps; j++) {
@@ -1873,6 +2020,22 @@ public:
         PSV_CU(launch_zero_planes<T>(memz.as<T>(), mz_shot, 0, mz_shot, B, st));
         PSV_CU(launch_zero_planes<T>(memx.as<T>(), mx_shot, 0, mx_shot, B, st));
         int rc = PSV_OK;
+        if (looped()) {  // no step boundaries on the stream: the steps' mean, in the velocity slot
+            for (int k = 0; k < 6; k++) ms6[k] = 0.0;
+            for (int pass = 0; pass < 2 && rc == PSV_OK; pass++) {
+                const bool adj = pass == 1;
+                cudaEventRecord(e[0], st);
+                rc = loop_steps(sp, adj ? qa : qf, adj ? MODE_ADJ : MODE_FWD, false, adj ? nt - 1 : 0,
+                                adj ? -1 : 1, nsteps, true, 0, ckpt ? nslots : sv.snt, nlaunch);
+                cudaEventRecord(e[1], st);
+                if (rc == PSV_OK) rc = sync_check();
+                float ms = 0;
+                if (rc == PSV_OK) cudaEventElapsedTime(&ms, e[0], e[1]);
+                ms6[pass * 3 + 1] = ms / nsteps;
+            }
+            for (auto &x : e) cudaEventDestroy(x);
+            return rc;
+        }
         for (int pass = 0; pass < 2 && rc == PSV_OK; pass++) {
             const bool adj = pass == 1;
             const SrcRecParams<T> &q = adj ? qa : qf;
@@ -1946,7 +2109,7 @@ public:
                 for (int t = 0; t < sv.snt; t++)
                     for (int jz = 0; jz < sv.snz; jz++)
                         for (int jx = 0; jx < sv.snx; jx++)
-                            h[(size_t)t * NHIST * snp + map[k] * snp + (size_t)jz * snx_pitch + jx] =
+                            h[(size_t)t * NHIST * snp + map[k] * snp + (size_t)jz * snx_pitch + snx_off + jx] =
                                 (T)accu_io[k][((size_t)t * sv.snz + jz) * sv.snx + jx];
             PSV_CU(cudaMemcpyAsync(hist.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
             PSV_CU(cudaStreamSynchronize(st));
@@ -2013,7 +2176,7 @@ public:
                         for (int jz = 0; jz < sv.snz; jz++)
                             for (int jx = 0; jx < sv.snx; jx++)
                                 accu_io[k][((size_t)t * sv.snz + jz) * sv.snx + jx] =
-                                    (double)h[(size_t)t * NHIST * snp + map[k] * snp + (size_t)jz * snx_pitch + jx] * un;
+                                    (double)h[(size_t)t * NHIST * snp + map[k] * snp + (size_t)jz * snx_pitch + snx_off + jx] * un;
         }
         if (grad_) {
             std::vector<T> h((size_t)gshot_shot);
@@ -2023,7 +2186,7 @@ public:
                     for (int jz = 0; jz < sv.snz; jz++)
                         for (int jx = 0; jx < sv.snx; jx++)
                             grad_out[k][(size_t)jz * sv.snx + jx] =
-                                (double)h[k * snp + (size_t)jz * snx_pitch + jx] * (k < 2 ? un / gscale : un) *
+                                (double)h[k * snp + (size_t)jz * snx_pitch + snx_off + jx] * (k < 2 ? un / gscale : un) *
                                 (g.imaging_sign > 0 ? -1.0 : 1.0);
         }
         return PSV_OK;

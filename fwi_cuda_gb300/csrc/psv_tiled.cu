@@ -494,16 +494,16 @@ PFN_cuTensorMapEncodeTiled_v12000 encoder()
 }  // namespace
 
 // 3-D map (column, row, plane) over nplanes planes of nz x nx floats with
-// row pitch `pitch` and plane stride `plane` elements; box bx x by x 1,
+// row pitch `pitch` and plane stride `plane` elements; box bx x by x bp,
 // zero fill outside.
 int encode3(CUtensorMap *map, const float *base, int nx, int nz, int pitch, long long plane,
-            int nplanes, int bx, int by)
+            int nplanes, int bx, int by, int bp)
 {
     auto encode = encoder();
     if (!encode) return fail(PSV_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     const cuuint64_t dim[3] = {(cuuint64_t)nx, (cuuint64_t)nz, (cuuint64_t)nplanes};
     const cuuint64_t stride[2] = {(cuuint64_t)pitch * 4, (cuuint64_t)plane * 4};
-    const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, (cuuint32_t)bp};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, (void *)base, dim, stride, box,
                               estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,

@@ -10,7 +10,7 @@
 namespace psv {
 namespace {
 
-constexpr unsigned WAIT_LIMIT = 1u << 20;  // try_wait rounds before giving up
+constexpr unsigned long long WAIT_LIMIT_NS = 2000000000ull;  // a wait gives up after two seconds
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p)
 {
@@ -48,19 +48,36 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes)
                  : "memory");
 }
 
+__device__ __forceinline__ unsigned long long now_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t)::"memory");
+    return t;
+}
+
+// Whether barrier `bar` has completed phase `parity`; may suspend the thread
+// for a while first.
+__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+
+// Bounded wait: by the clock, because one try may suspend for milliseconds.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity)
 {
-    for (unsigned n = 0; n < WAIT_LIMIT; n++) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred P;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P;\n\t}"
-            : "=r"(done)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
+    if (mbar_try(bar, parity)) return true;
+    const unsigned long long t0 = now_ns();
+    do {
+        if (mbar_try(bar, parity)) return true;
+    } while (now_ns() - t0 < WAIT_LIMIT_NS);
     return false;
 }
 

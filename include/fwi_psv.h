@@ -52,7 +52,9 @@ typedef enum {
 
 /* Time-step kernel families (psv_options.kernel_family). */
 #define PSV_KERNELS_DIRECT 1    /* per-thread loads of the stencil neighbours */
-#define PSV_KERNELS_TMA 2       /* tiles staged in shared memory by TMA tensor copies (FP32) */
+#define PSV_KERNELS_TMA 2       /* tiles staged in shared memory by TMA tensor copies; up to
+                                   hundreds of time steps per launch with no free surface or a
+                                   top one whose mirrored rows fit the first tile (FP32) */
 #define PSV_KERNELS_VEC4 3      /* four columns per thread, 128-bit loads and stores (FP32) */
 #define PSV_KERNELS_FUSED 4     /* one launch per time step: stress of a tile and its halo,
                                    then its velocities, from shared memory (FP32) */
@@ -151,7 +153,8 @@ typedef struct psv_options {
                                    warp-shuffle variant); TMA family 2, 4, 8; VEC4 family
                                    1, 2, 4; FUSED family: tile rows 16 or 32; MARCH family:
                                    rows each CTA marches, 32, 64 or 128; 0 = default */
-    int kernel_family;          /* time-step kernels: 0 = any (the autotuner chooses),
+    int kernel_family;          /* time-step kernels: 0 = any (the autotuner chooses; before
+                                   and without it, by the batch's grid points),
                                    PSV_KERNELS_DIRECT, _TMA, _VEC4, _FUSED or _MARCH (the
                                    last four FP32 only; FUSED needs no free surface but a top
                                    one, MARCH none or a top one on the first interior row) */
