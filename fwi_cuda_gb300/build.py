@@ -34,6 +34,7 @@ UNITS = [
     ("psv_kernels_f64.cu", []),
     ("psv_tiled.cu", []),
     ("psv_loop.cu", []),
+    ("psv_resident.cu", []),
     ("psv_vec.cu", []),
     ("psv_fused.cu", []),
     ("psv_march.cu", []),

@@ -277,8 +277,18 @@ int psv_gradient(psv_plan *p, double *L2, double *gl, double *gm, double *gr)
     return PSV_OK;
 }
 
+// Several plans are about to run at once.
+static int share_all(psv_plan *const *plans, int n)
+{
+    if (plans && n > 1)
+        for (int k = 0; k < n; k++)
+            if (plans[k] && plans[k]->impl) PSV_TRY(plans[k]->impl->share());
+    return PSV_OK;
+}
+
 int psv_multi_forward(psv_plan *const *plans, int n, double *const *uz, double *const *ux)
 {
+    PSV_TRY(share_all(plans, n));
     return run_plans(plans, n, [&](int k) {
         return plans[k]->impl->forward(uz ? uz[k] : nullptr, ux ? ux[k] : nullptr);
     });
@@ -286,6 +296,7 @@ int psv_multi_forward(psv_plan *const *plans, int n, double *const *uz, double *
 
 int psv_multi_gradient(psv_plan *const *plans, int n, double *L2)
 {
+    PSV_TRY(share_all(plans, n));
     if (plans && n > 0)
         for (int k = 0; k < n; k++)  // tune serially: concurrent work would distort the timings
             if (plans[k] && plans[k]->impl) PSV_TRY(plans[k]->impl->prepare());

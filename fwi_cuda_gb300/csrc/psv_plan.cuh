@@ -72,6 +72,14 @@ int encode_loop_maps(LoopMaps *m, const float *fld, int nfplanes, int nx, int nz
                      int ngplanes, int snx_pitch, int snz);
 cudaError_t launch_loop(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopMaps &m,
                         const LoopRun &run, int ns, int mode, int tz, int nbatch, cudaStream_t st);
+// The same steps with the wavefields on chip, for batches that fit (FP32,
+// psv_resident.cu): one tile of 32 columns x tz rows per CTA.  run.keep by
+// tiles of 64 x 16; run.sync: resident_inbox_bytes.  resident_rows: tz, 0 if
+// the batch does not fit the GPU's SMs or its surfaces cross tiles.
+int resident_rows(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm);
+size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, int tz);
+cudaError_t launch_resident(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopRun &run, int ns,
+                            int mode, int tz, int nbatch, cudaStream_t st);
 // Four-columns-per-thread kernels (FP32, psv_vec.cu): blocks of 32 x by
 // threads over 128 columns x by * rpt rows, rpt in {1, 2, 4}.
 cudaError_t launch_stress_v4(const StepParams<float> &p, int ns, int rpt, int by, int nbatch,
@@ -256,6 +264,7 @@ struct PlanIface {
     virtual void shape(int *fam, int *rpt, int *by) const = 0;
     virtual void storage(int *kind, int *segment_steps, int *slots, long long *advances) const = 0;
     virtual int chain_count() const = 0;
+    virtual int share() = 0;    // other plans run at the same time (psv_multi_*)
     virtual int prepare() = 0;  // history buffers and the pending autotune, before concurrent use
     // Joint forward modelling (psv_joint.cu): switch to the direct family with
     // rpt rows per thread and 32 x by blocks, select shot batch `batch`, zero

@@ -69,7 +69,8 @@ public:
     int fam = PSV_KERNELS_DIRECT;                    // kernel family of the time step
     TileMaps tmap{}, tmap2{};                        // tensor maps of fld / fld2 (TMA family)
     LoopMaps lmap{}, lmap2{};                        // ... and of its many-step launches
-    DevMem lsync;                                    // their item counter and progress words
+    int rz = 0;                                      // tile rows of the resident kernel (0: does not serve)
+    DevMem lsync;                                    // item counter and progress words, or the tiles' inboxes
     DevMem lkeep, lkept;                             // per tile: keeps its sums' roundings; those tiles
     int nkept = 0;
     long long ck_kept = 0;  // elements of a checkpointed state that hold them
@@ -102,6 +103,7 @@ public:
     double t_ms[3] = {0, 0, 0};
     bool have_model = false, have_obs = false, store_flag = false;
     bool tuned = false;
+    bool beside = false;  // runs at the same time as other plans (psv_multi_*)
     long long nlaunch = 0;          // kernels launched (graph nodes counted per replay)
     long long gx_nodes[NPASS] = {}; // kernels in each captured pass
     dim3 blk{32, 8, 1};
@@ -310,16 +312,14 @@ public:
         }
         if (ckpt) hist_shot = (long long)nslots * NHIST * snap_plane;
         nbatch = (nshot + B - 1) / B;
-        // The shape of a plan nobody autotunes (modelling).  From 500 000
-        // points in a batch the looped TMA tiles beat the direct kernels:
-        // 12.7 against 14.1 us a step at 0.54 M points (301 x 601, 3 shots,
-        // order 4), 16.5 against 25.9 at 1.4 M, 21 against 40 at 2.0 M
-        // (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
-        if (sizeof(T) == 4 && opt.kernel_family == 0 && opt.rows_per_thread == 0 && opt.block_y <= 0 &&
-            (double)nz * nx * B >= 500e3 && loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
-            fam = PSV_KERNELS_TMA;
-            rpt = 4;
+        if (sizeof(T) == 4) {
+            int dev = 0, nsm = 0, coop = 0;
+            PSV_CU(cudaGetDevice(&dev));
+            PSV_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+            PSV_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+            rz = coop ? resident_rows(nz, nx, B, sv.ns, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1, nsm) : 0;
         }
+        if (any_kernels()) fam = start_shape(&rpt);
 
         PSV_CU(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         for (auto &e : ev) PSV_CU(cudaEventCreate(&e));
@@ -350,7 +350,8 @@ public:
         PSV_TRY(traces.alloc((size_t)6 * nshot * ntr * 8 + 8, total));
         PSV_TRY(red.alloc(((size_t)256 * std::max(3, nshot) + nshot + 3 + B + 2) * 8, total));
         PSV_TRY(taperb.alloc((size_t)(nx + nz) * 8, total));
-        if (sizeof(T) == 4) PSV_TRY(lsync.alloc(loop_sync_bytes(nz, nx, B), total));
+        if (sizeof(T) == 4) PSV_TRY(lsync.alloc(std::max(loop_sync_bytes(nz, nx, B),
+                                                           rz ? resident_inbox_bytes(nz, nx, B, sv.ns, rz) : 0), total));
         PSV_TRY(ctl.alloc(4 * sizeof(int), total));
         PSV_TRY(ctl2.alloc(2 * MAXCH * sizeof(int), total));
         PSV_CU(cudaMemsetAsync(ctl2.p, 0, 2 * MAXCH * sizeof(int), st));
@@ -400,11 +401,16 @@ public:
     // Many steps per launch (psv_loop.cu): the TMA family, except with bottom or
     // side surfaces or mirrored rows beyond the first tile, whose mirror writes
     // cross tiles (those step through psv_tiled.cu).
+    // Eight rows per thread stand for the kernel that keeps the wavefields on
+    // chip (psv_resident.cu) where it serves, else for 32-row tiles of
+    // psv_tiled.cu.
+    bool resident() const { return sizeof(T) == 4 && fam == PSV_KERNELS_TMA && rpt == 8 && rz; }
     bool looped() const
     {
-        return sizeof(T) == 4 && fam == PSV_KERNELS_TMA &&
-               loop_supported(4 * rpt, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1);
+        return resident() || (sizeof(T) == 4 && fam == PSV_KERNELS_TMA &&
+                              loop_supported(4 * rpt, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1));
     }
+    int kept_rows() const { return resident() ? 16 : 4 * rpt; }  // rows of a tile of kept_tiles()
     // Snapshot slots per shot that a tensor map of the history covers (0: none,
     // not allocated or the window is subsampled).
     int image_slots() const
@@ -433,7 +439,7 @@ public:
     {
         nkept = 0;
         if (!looped()) return PSV_OK;
-        const int tz = 4 * rpt;
+        const int tz = kept_rows();
         const std::vector<int> t = kept_tiles(tz);
         std::vector<int> on((size_t)((sv.g.nx + 63) / 64) * ((sv.g.nz + tz - 1) / tz), 0);
         for (int k : t) on[(size_t)k] = 1;
@@ -449,7 +455,7 @@ public:
         if constexpr (sizeof(T) == 4)
             if (looped())
                 return launch_loop_kept(op, s.fld + (long long)s.pp_planes * plane, s.shot_stride, plane, pitch,
-                                        sv.g.nz, sv.g.nx, 4 * rpt, lkept.as<int>(), nkept,
+                                        sv.g.nz, sv.g.nx, kept_rows(), lkept.as<int>(), nkept,
                                         state ? state + ck_state - ck_kept : nullptr, ck_state, B, st);
         return cudaSuccess;
     }
@@ -467,7 +473,8 @@ public:
                 const LoopRun run{std::min(most, n - j), it0 + j * dit, dit, sv.g.snap_dt, base,
                                   std::max(ring, 1), snap, far, mode == MODE_ADJ ? image_slots() : 0,
                                   nkept ? lkeep.as<int>() : nullptr, lsync.as<int>()};
-                PSV_CU(launch_loop(s, q, second ? lmap2 : lmap, run, sv.ns, mode, 4 * rpt, B, st));
+                if (resident()) PSV_CU(launch_resident(s, q, run, sv.ns, mode, rz, B, st));
+                else PSV_CU(launch_loop(s, q, second ? lmap2 : lmap, run, sv.ns, mode, 4 * rpt, B, st));
                 nk++;
             }
         }
@@ -477,6 +484,41 @@ public:
     // (the fused family ping-pongs; the others update in place, copy 0).
     int par(int k) const { return fused() ? (k & 1) : 0; }
     static int v4_rpt(int r) { return (r == 1 || r == 2 || r == 4) ? r : 1; }
+
+    // Whether the plan may choose its kernels.
+    bool any_kernels() const { return opt.kernel_family == 0 && opt.rows_per_thread == 0; }
+    // The shape of a plan nobody autotunes (modelling).  The resident kernel
+    // where the batch fits it (a block shape given is the direct family's); from 500 000 points in a batch the looped TMA
+    // tiles beat the direct kernels: 12.7 against 14.1 us a step at 0.54 M
+    // points (301 x 601, 3 shots, order 4), 16.5 against 25.9 at 1.4 M, 21
+    // against 40 at 2.0 M (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
+    int start_shape(int *r) const
+    {
+        if (rz && !beside && opt.chains == 0) {
+            *r = 8;
+            return PSV_KERNELS_TMA;
+        }
+        if (sizeof(T) == 4 && opt.block_y <= 0 && (double)sv.g.nz * sv.g.nx * B >= 500e3 &&
+            loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
+            *r = 4;
+            return PSV_KERNELS_TMA;
+        }
+        *r = 1;
+        return PSV_KERNELS_DIRECT;
+    }
+    // Runs beside other plans from now on.  The resident kernel waits until
+    // the GPU has room for all its CTAs and shares it with nobody else that
+    // fills it: four surveys at once took 21.3 ms with it, 16.6 with kernels
+    // that mix.
+    int share() override
+    {
+        if (beside || !any_kernels()) return PSV_OK;
+        beside = true;
+        if (!resident()) return PSV_OK;
+        tuned = false;
+        int r, f = start_shape(&r);
+        return set_shape(f, r, opt.block_y > 0 ? opt.block_y : 8);
+    }
 
     // Tensor maps of the field blocks for the TMA family (rebuilt when the
     // tile height or a field buffer changes).
@@ -492,7 +534,7 @@ public:
                                               pitch, plane, sv.ns, (int)blk.y));
                 return PSV_OK;
             }
-            if (fam != PSV_KERNELS_TMA) return PSV_OK;
+            if (fam != PSV_KERNELS_TMA || resident()) return PSV_OK;
             PSV_TRY(encode_tile_maps(&tmap, fld.as<float>(), (int)(B * nfield()), coef.as<float>(),
                                      g.nx, g.nz, pitch, plane, sv.ns, rpt));
             if (looped())
@@ -707,7 +749,7 @@ public:
     }
 
     // Sources and receivers bucketed by the velocity kernel's tiles (direct
-    // family: 32 columns x blk.y * |rpt| rows; TMA: 64 x 4 rpt; VEC4: 128 x
+    // family: 32 columns x blk.y * |rpt| rows; TMA: 64 x 4 rpt, resident 32 x rz; VEC4: 128 x
     // blk.y * rpt; FUSED: 64 x rpt; MARCH: 32 blk.y - fdorder x rpt), so each
     // block finds its own.
     int build_tile_index()
@@ -715,8 +757,8 @@ public:
         const int nshot = sv.s.nshot, nrec = sv.s.nrec;
         const bool tma = fam == PSV_KERNELS_TMA, v4 = fam == PSV_KERNELS_VEC4;
         const bool mr = fam == PSV_KERNELS_MARCH;
-        const int tw = mr ? march_tile_width(sv.ns, (int)blk.y) : tma || fused() ? 64 : v4 ? 128 : 32;
-        const int tz = tma ? 4 * rpt : fused() ? rpt : (int)blk.y * (rpt < 0 ? -rpt : rpt);
+        const int tw = mr ? march_tile_width(sv.ns, (int)blk.y) : resident() ? 32 : tma || fused() ? 64 : v4 ? 128 : 32;
+        const int tz = resident() ? rz : tma ? 4 * rpt : fused() ? rpt : (int)blk.y * (rpt < 0 ? -rpt : rpt);
         const int ntx = (sv.g.nx + tw - 1) / tw, ntz = (sv.g.nz + tz - 1) / tz;
         const int nt_ = ntx * ntz;
         auto tile_of = [&](int z, int x) { return (z / tz) * ntx + x / tw; };
@@ -1645,7 +1687,8 @@ public:
     {
         // (plans the loops cannot serve choose among other kernels)
         const TuneKey key{sv.g.nz, sv.g.nx, sv.ns, B, (int)sizeof(T),
-                          opt.kernel_family + (loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) ? 0 : 16)};
+                          opt.kernel_family + (loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) ? 0 : 16) +
+                              (rz && !beside ? 32 : 0)};
         auto report = [&] {
             if (out_fam) *out_fam = fam;
             if (out_rpt) *out_rpt = rpt;
@@ -1673,7 +1716,9 @@ public:
             }
         }
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_TMA))
-            for (int r : {2, 4}) cand.emplace_back(PSV_KERNELS_TMA, r, 4);
+            for (int r : {2, 4, 8})  // (8: on chip or two launches a step, the latter where no loop serves)
+                if (r < 8 || (rz ? !beside : !loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)))
+                    cand.emplace_back(PSV_KERNELS_TMA, r, 4);
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_VEC4))
             for (int r : {1, 2, 4})
                 for (int by : {2, 4, 8}) cand.emplace_back(PSV_KERNELS_VEC4, r, by);
