@@ -73,13 +73,16 @@ int encode_loop_maps(LoopMaps *m, const float *fld, int nfplanes, int nx, int nz
 cudaError_t launch_loop(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopMaps &m,
                         const LoopRun &run, int ns, int mode, int tz, int nbatch, cudaStream_t st);
 // The same steps with the wavefields on chip, for batches that fit (FP32,
-// psv_resident.cu): one tile of 32 columns x tz rows per CTA.  run.keep by
-// tiles of 64 x 16; run.sync: resident_inbox_bytes.  resident_rows: tz, 0 if
-// the batch does not fit the GPU's SMs or its surfaces cross tiles.
-int resident_rows(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm);
-size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, int tz);
+// psv_resident.cu): one tile of rw columns (32 or 64) x tz rows per CTA.
+// run.keep by tiles of 64 x 16; run.sync: resident_inbox_bytes.  resident_tile:
+// tz = 0 if the batch does not fit the GPU's SMs or its surfaces cross tiles.
+struct ResidentTile {
+    int rw, tz;
+};
+ResidentTile resident_tile(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm);
+size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, const ResidentTile &t);
 cudaError_t launch_resident(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopRun &run, int ns,
-                            int mode, int tz, int nbatch, cudaStream_t st);
+                            int mode, const ResidentTile &t, int nbatch, cudaStream_t st);
 // Four-columns-per-thread kernels (FP32, psv_vec.cu): blocks of 32 x by
 // threads over 128 columns x by * rpt rows, rpt in {1, 2, 4}.
 cudaError_t launch_stress_v4(const StepParams<float> &p, int ns, int rpt, int by, int nbatch,

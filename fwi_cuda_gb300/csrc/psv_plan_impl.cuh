@@ -69,7 +69,7 @@ public:
     int fam = PSV_KERNELS_DIRECT;                    // kernel family of the time step
     TileMaps tmap{}, tmap2{};                        // tensor maps of fld / fld2 (TMA family)
     LoopMaps lmap{}, lmap2{};                        // ... and of its many-step launches
-    int rz = 0;                                      // tile rows of the resident kernel (0: does not serve)
+    ResidentTile rt{};                               // tiles of the resident kernel (tz = 0: does not serve)
     DevMem lsync;                                    // item counter and progress words, or the tiles' inboxes
     DevMem lkeep, lkept;                             // per tile: keeps its sums' roundings; those tiles
     int nkept = 0;
@@ -317,7 +317,7 @@ public:
             PSV_CU(cudaGetDevice(&dev));
             PSV_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
             PSV_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-            rz = coop ? resident_rows(nz, nx, B, sv.ns, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1, nsm) : 0;
+            if (coop) rt = resident_tile(nz, nx, B, sv.ns, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1, nsm);
         }
         if (any_kernels()) fam = start_shape(&rpt);
 
@@ -351,7 +351,7 @@ public:
         PSV_TRY(red.alloc(((size_t)256 * std::max(3, nshot) + nshot + 3 + B + 2) * 8, total));
         PSV_TRY(taperb.alloc((size_t)(nx + nz) * 8, total));
         if (sizeof(T) == 4) PSV_TRY(lsync.alloc(std::max(loop_sync_bytes(nz, nx, B),
-                                                           rz ? resident_inbox_bytes(nz, nx, B, sv.ns, rz) : 0), total));
+                                                           rt.tz ? resident_inbox_bytes(nz, nx, B, sv.ns, rt) : 0), total));
         PSV_TRY(ctl.alloc(4 * sizeof(int), total));
         PSV_TRY(ctl2.alloc(2 * MAXCH * sizeof(int), total));
         PSV_CU(cudaMemsetAsync(ctl2.p, 0, 2 * MAXCH * sizeof(int), st));
@@ -404,7 +404,7 @@ public:
     // Eight rows per thread stand for the kernel that keeps the wavefields on
     // chip (psv_resident.cu) where it serves, else for 32-row tiles of
     // psv_tiled.cu.
-    bool resident() const { return sizeof(T) == 4 && fam == PSV_KERNELS_TMA && rpt == 8 && rz; }
+    bool resident() const { return sizeof(T) == 4 && fam == PSV_KERNELS_TMA && rpt == 8 && rt.tz; }
     bool looped() const
     {
         return resident() || (sizeof(T) == 4 && fam == PSV_KERNELS_TMA &&
@@ -473,7 +473,7 @@ public:
                 const LoopRun run{std::min(most, n - j), it0 + j * dit, dit, sv.g.snap_dt, base,
                                   std::max(ring, 1), snap, far, mode == MODE_ADJ ? image_slots() : 0,
                                   nkept ? lkeep.as<int>() : nullptr, lsync.as<int>()};
-                if (resident()) PSV_CU(launch_resident(s, q, run, sv.ns, mode, rz, B, st));
+                if (resident()) PSV_CU(launch_resident(s, q, run, sv.ns, mode, rt, B, st));
                 else PSV_CU(launch_loop(s, q, second ? lmap2 : lmap, run, sv.ns, mode, 4 * rpt, B, st));
                 nk++;
             }
@@ -494,7 +494,7 @@ public:
     // against 40 at 2.0 M (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
     int start_shape(int *r) const
     {
-        if (rz && !beside && opt.chains == 0) {
+        if (rt.tz && !beside && opt.chains == 0) {
             *r = 8;
             return PSV_KERNELS_TMA;
         }
@@ -749,7 +749,7 @@ public:
     }
 
     // Sources and receivers bucketed by the velocity kernel's tiles (direct
-    // family: 32 columns x blk.y * |rpt| rows; TMA: 64 x 4 rpt, resident 32 x rz; VEC4: 128 x
+    // family: 32 columns x blk.y * |rpt| rows; TMA: 64 x 4 rpt, resident rt; VEC4: 128 x
     // blk.y * rpt; FUSED: 64 x rpt; MARCH: 32 blk.y - fdorder x rpt), so each
     // block finds its own.
     int build_tile_index()
@@ -757,8 +757,8 @@ public:
         const int nshot = sv.s.nshot, nrec = sv.s.nrec;
         const bool tma = fam == PSV_KERNELS_TMA, v4 = fam == PSV_KERNELS_VEC4;
         const bool mr = fam == PSV_KERNELS_MARCH;
-        const int tw = mr ? march_tile_width(sv.ns, (int)blk.y) : resident() ? 32 : tma || fused() ? 64 : v4 ? 128 : 32;
-        const int tz = resident() ? rz : tma ? 4 * rpt : fused() ? rpt : (int)blk.y * (rpt < 0 ? -rpt : rpt);
+        const int tw = mr ? march_tile_width(sv.ns, (int)blk.y) : resident() ? rt.rw : tma || fused() ? 64 : v4 ? 128 : 32;
+        const int tz = resident() ? rt.tz : tma ? 4 * rpt : fused() ? rpt : (int)blk.y * (rpt < 0 ? -rpt : rpt);
         const int ntx = (sv.g.nx + tw - 1) / tw, ntz = (sv.g.nz + tz - 1) / tz;
         const int nt_ = ntx * ntz;
         auto tile_of = [&](int z, int x) { return (z / tz) * ntx + x / tw; };
@@ -1688,7 +1688,7 @@ public:
         // (plans the loops cannot serve choose among other kernels)
         const TuneKey key{sv.g.nz, sv.g.nx, sv.ns, B, (int)sizeof(T),
                           opt.kernel_family + (loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) ? 0 : 16) +
-                              (rz && !beside ? 32 : 0)};
+                              (rt.tz && !beside ? 32 : 0)};
         auto report = [&] {
             if (out_fam) *out_fam = fam;
             if (out_rpt) *out_rpt = rpt;
@@ -1717,7 +1717,7 @@ public:
         }
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_TMA))
             for (int r : {2, 4, 8})  // (8: on chip or two launches a step, the latter where no loop serves)
-                if (r < 8 || (rz ? !beside : !loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)))
+                if (r < 8 || (rt.tz ? !beside : !loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)))
                     cand.emplace_back(PSV_KERNELS_TMA, r, 4);
         if (sizeof(T) == 4 && (opt.kernel_family == 0 || opt.kernel_family == PSV_KERNELS_VEC4))
             for (int r : {1, 2, 4})

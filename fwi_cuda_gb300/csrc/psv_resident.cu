@@ -5,9 +5,10 @@
 // between SMs, not on arithmetic: two launches cost 9 to 12 us a step however
 // small the grid, the tile list of psv_loop.cu 11 to 12 (claim, load, store,
 // fence and progress word of each half-step).  Here a CTA keeps one tile of
-// 32 columns x tz rows of one shot for the whole launch: v, sigma and their
-// halos in shared memory, u, We and the CPML memories in registers, one quad
-// of columns per thread.  Only the tiles' rims travel, once per half-step.
+// 32 or 64 columns x tz rows of one shot for the whole launch: v, sigma and
+// their halos in shared memory, u and We in registers, one or two quads of
+// columns per thread; the CPML memories in registers with one quad, through L1
+// with two.  Only the tiles' rims travel, once per half-step.
 //
 // A rim cell is sent as two 64-bit words {value, half-step number}, written by
 // one 128-bit store straight into the neighbour's inbox and polled there: a
@@ -17,11 +18,13 @@
 // own next rim has arrived here, which it sends after reading the cell.
 //
 // What bounds it: the rim's way, about 1 us of each half-step, and the chain
-// of one quad's update behind it.  us a step forward / adjoint, two direct
-// launches (event-timed passes) before -> here:
-//   101 x 201, 1 shot, order 4    9.0 / -    -> 3.0 / 3.2   (tiles of 8 rows)
-//   301 x 601, 1 shot, order 4    11 / 12    -> 3.8 / 4.2   (38)
-//   187 x 133, 5 shots, order 6   10 / 11    -> 4.0 / 4.2   (32)
+// of a quad's update behind it.  us a step forward / adjoint:
+//   101 x 201, 1 shot, order 4    2.9 / 3.1   (tiles of 32 x 8)
+//   301 x 601, 1 shot, order 4    3.6 / 4.0   (32 x 38)
+//   281 x 561, 2 shots, order 4   6.9 / 8.0   (64 x 36; 13.1 / 14.6 by psv_loop.cu)
+// and whole passes, two launches a step before -> here: 400 steps of modelling
+// on the first grid 3676 -> 1377 us, the second's gradient (800 steps)
+// 9292 -> 4680, five shots on 187 x 133, order 6, 1000 steps 10595 -> 4627.
 // What neither the next update nor a neighbour waits for comes after the rim
 // of v is sent: snapshots, imaging, traces; source amplitudes are fetched
 // before the waits.  The traces' FP64 divide, at a 64th of the FP32 rate, held
@@ -29,7 +32,7 @@
 // that order, took 400 steps of modelling on 101 x 201 from 1916 to 1378 us.
 //
 // All CTAs must be resident: the launch is cooperative, one CTA or more per SM
-// (resident_rows).  Waits are bounded: after two seconds StepParams::err is set
+// (resident_tile).  Waits are bounded: after two seconds StepParams::err is set
 // and the CTA leaves; the host turns that into PSV_ERR_CUDA.
 #include <algorithm>
 
@@ -41,28 +44,28 @@ namespace psv {
 
 namespace {
 
-constexpr int RW = 32;           // tile columns
-constexpr int RS = RW + 2 * HX;  // staged row length (floats)
 constexpr int MAX_THREADS = 512;
 
+// rw: tile columns, 32 or 64.
+__host__ __device__ constexpr int staged_row(int rw) { return rw + 2 * HX; }
 // Cells of a tile's rim: NS rows above and below, NS columns left and right.
-__host__ __device__ constexpr int rim_cells(int ns, int tz) { return 2 * ns * (RW + tz); }
-// One quad per thread, and at most two rim cells.
-__host__ __device__ constexpr int resident_threads(int ns, int tz)
+__host__ __device__ constexpr int rim_cells(int ns, int rw, int tz) { return 2 * ns * (rw + tz); }
+// Eight threads to a row, and at most two rim cells to a thread.
+__host__ __device__ constexpr int resident_threads(int ns, int rw, int tz)
 {
-    const int q = RW / 4 * tz, r = rim_cells(ns, tz);
+    const int q = 8 * tz, r = rim_cells(ns, rw, tz);
     const int n = q > r ? q : r < MAX_THREADS ? r : MAX_THREADS;
     return (n + 31) / 32 * 32;
 }
 // v and sigma with halo, and what the sums of five fields kept.
-__host__ __device__ constexpr int resident_smem(int ns, int tz)
+__host__ __device__ constexpr int resident_smem(int ns, int rw, int tz)
 {
-    return 4 * (5 * (tz + 2 * ns) * RS + 5 * tz * RW);
+    return 4 * (5 * (tz + 2 * ns) * staged_row(rw) + 5 * tz * rw);
 }
 
 struct ResidentRun {
     LoopRun r;
-    int tz, ntx, ntz;
+    int tz, ntx, ntz;  // rows of a tile, tiles
     ulonglong2 *inbox;  // [tile][v, sigma][rim cell]
 };
 
@@ -90,65 +93,92 @@ struct Rim {
     bool x;             // left or right face: sigma's planes szx, sxx instead of szz, szx
 };
 
-// The tile's quad of a strip's memory planes, if it lies in the strip.
-struct Strip {
-    float *z, *x;  // null: outside
+// A quad of the thread: columns ix .. ix + 3 of the tile's row.
+struct Quad {
+    int ix;
+    bool mine, keep;  // on the grid; its sums keep their roundings
+    unsigned mask;    // interior columns
+    float *z, *x;     // in the z and x strips' memories, null outside
+    Q4 we, uz, ux;
+    Q4 mz[4], mx[4];  // CPML memories of a thread with one quad
 };
 
-template <int NS, int MODE>
+// CPML of one derivative: memory `o` in registers where the thread has one
+// quad, else through L1 (only this thread reads and writes it in the launch).
+template <int QPT>
+__device__ __forceinline__ void cpml_at(Q4 &o, float *m, const Q4 &a, const Q4 &b, const Q4 &ki, Q4 &d, unsigned mask)
+{
+    if constexpr (QPT > 1) o = lds4(m);
+    cpml_quad(o, a, b, ki, d, mask);
+    if constexpr (QPT > 1) st4(m, o);
+}
+
+template <int NS, int QPT, int MODE>
 __global__ void __launch_bounds__(MAX_THREADS, 1)
     k_resident(const __grid_constant__ StepParams<float> p, const __grid_constant__ SrcRecParams<float> q,
                const __grid_constant__ ResidentRun g)
 {
     constexpr bool U = has_u<MODE>(), WE = has_we<MODE>(), FWD = MODE != MODE_ADJ;
+    constexpr int RW = 32 * QPT, RS = staged_row(RW);
     extern __shared__ __align__(16) float sm[];
     const LoopRun &run = g.r;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nthr = blockDim.x;
     const int c = blockIdx.x % g.ntx, bc = blockIdx.x / g.ntx, b = bc % g.ntz, bz = bc / g.ntz;
     if (bz >= p.ctl[1]) return;  // the last batch may hold fewer shots
-    const int tz = g.tz, HP = (tz + 2 * NS) * RS, KP = tz * RW, cells = rim_cells(NS, tz);
+    const int tz = g.tz, HP = (tz + 2 * NS) * RS, KP = tz * RW, cells = rim_cells(NS, RW, tz);
     const int x0 = c * RW, z0 = b * tz;
     float *sv = sm, *ss = sm + 2 * HP, *kept = sm + 5 * HP;
     const int lr = tid >> 3, qc = 4 * (tid & 7);
-    const int iz = z0 + lr, ix = x0 + qc;
-    const bool mine = lr < tz && iz < p.nz && ix < p.nx;
-    const unsigned mask = mine && iz >= p.nz1 && iz < p.nz2 ? inner_mask(p, ix) : 0;
-    const int o = (lr + NS) * RS + HX + qc;  // the quad in a staged plane
-    const int ko = lr * RW + qc;             // ... and in a plane of kept roundings
-    const int i = iz * p.pitch + ix;
-    float *f = p.fld + (long long)bz * p.shot_stride + i;
-    float *fk = f + (long long)p.pp_planes * p.plane;  // kept roundings between launches
-    const bool keep = FWD && mine && run.keep && run.keep[iz / 16 * ((p.nx + 63) / 64) + ix / 64];
+    const int iz = z0 + lr;
+    const int o0 = (lr + NS) * RS + HX + qc;  // the first quad in a staged plane; the next 32 columns on
+    const int ko0 = lr * RW + qc;             // ... and in a plane of kept roundings
+    float *fs = p.fld + (long long)bz * p.shot_stride;
+    float *fk = fs + (long long)p.pp_planes * p.plane;  // kept roundings between launches
+    Quad quad[QPT];
+#pragma unroll
+    for (int j = 0; j < QPT; j++) {
+        Quad &t = quad[j];
+        t.ix = x0 + qc + 32 * j;
+        t.mine = lr < tz && iz < p.nz && t.ix < p.nx;
+        t.mask = t.mine && iz >= p.nz1 && iz < p.nz2 ? inner_mask(p, t.ix) : 0;
+        t.keep = FWD && t.mine && run.keep && run.keep[iz / 16 * ((p.nx + 63) / 64) + t.ix / 64];
+        t.z = t.x = nullptr;
+        t.we = t.uz = t.ux = all4(0.f);
+    }
 
     // ---- what stays on chip, from the field block
     for (int e = tid; e < 5 * HP + 5 * KP; e += nthr) sm[e] = 0.f;
     __syncthreads();
-    Q4 we = all4(0.f), uz = all4(0.f), ux = all4(0.f), mz[4], mx[4];
-    Strip strip{nullptr, nullptr};
-    if (mine) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) st4(sm + k * HP + o, ldg4(f + (F_VZ + k) * p.plane));
-        if (keep)
+    for (int j = 0; j < QPT; j++) {
+        Quad &t = quad[j];
+        const int o = o0 + 32 * j, ko = ko0 + 32 * j, i = iz * p.pitch + t.ix;
+        if (t.mine) {
 #pragma unroll
-            for (int k = 0; k < 5; k++) st4(kept + k * KP + ko, ldg4(fk + (F_VZ + k) * p.plane));
-        if constexpr (WE) we = ldg4(f + (FWD ? F_WE : F_WEA) * p.plane);
-        if constexpr (U) {
-            uz = ldg4(f + F_UZ * p.plane);
-            ux = ldg4(f + F_UX * p.plane);
+            for (int k = 0; k < 5; k++) st4(sm + k * HP + o, ldg4(fs + i + (F_VZ + k) * p.plane));
+            if (t.keep)
+#pragma unroll
+                for (int k = 0; k < 5; k++) st4(kept + k * KP + ko, ldg4(fk + i + (F_VZ + k) * p.plane));
+            if constexpr (WE) t.we = ldg4(fs + i + (FWD ? F_WE : F_WEA) * p.plane);
+            if constexpr (U) {
+                t.uz = ldg4(fs + i + F_UZ * p.plane);
+                t.ux = ldg4(fs + i + F_UX * p.plane);
+            }
         }
-    }
-    if (mask) {
+        if (!t.mask) continue;
         if (iz < p.pz0 || iz >= p.pz1) {
             const int rr = iz < p.pz0 ? iz : iz - p.pz1 + p.pz0;
-            strip.z = p.memz + (long long)bz * p.mz_shot_stride + (long long)rr * p.pitch + ix;
+            t.z = p.memz + (long long)bz * p.mz_shot_stride + (long long)rr * p.pitch + t.ix;
+            if constexpr (QPT == 1)
 #pragma unroll
-            for (int k = 0; k < 4; k++) mz[k] = ldg4(strip.z + k * p.mz_plane);
+                for (int k = 0; k < 4; k++) t.mz[k] = ldg4(t.z + k * p.mz_plane);
         }
-        if (ix < p.px0 || ix >= p.px1) {
-            const int cc = ix < p.px0 ? ix : ix - p.px1 + p.px0;
-            strip.x = p.memx + (long long)bz * p.mx_shot_stride + (long long)iz * p.mx_pitch + cc;
+        if (t.ix < p.px0 || t.ix >= p.px1) {
+            const int cc = t.ix < p.px0 ? t.ix : t.ix - p.px1 + p.px0;
+            t.x = p.memx + (long long)bz * p.mx_shot_stride + (long long)iz * p.mx_pitch + cc;
+            if constexpr (QPT == 1)
 #pragma unroll
-            for (int k = 0; k < 4; k++) mx[k] = ldg4(strip.x + k * p.mx_plane);
+                for (int k = 0; k < 4; k++) t.mx[k] = ldg4(t.x + k * p.mx_plane);
         }
     }
     // ---- the rim: faces above, below, left, right
@@ -288,14 +318,17 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
             ax = stx[(long long)it * q.stf_ncol + s0.col];
         }
         if constexpr (!FWD)
-            if (slot >= 0 && mine && p.snap_dx == 1) {
-                const int dzr = iz - p.snap_z1, w = ix - p.snap_x1;
-                if (dzr >= 0 && iz <= p.snap_z2 && dzr % p.snap_dz == 0 && w >= 0 && ix <= p.snap_x2) {
-                    const float *h = p.hist + (long long)bz * p.hist_shot_stride +
-                                     (long long)slot * p.hist_slot_stride + (long long)(dzr / p.snap_dz) * p.snx_pitch + w;
+            if (slot >= 0 && p.snap_dx == 1) {
+                const int dzr = iz - p.snap_z1;
+                const float *row = p.hist + (long long)bz * p.hist_shot_stride + (long long)slot * p.hist_slot_stride +
+                                   (long long)(dzr / p.snap_dz) * p.snx_pitch;
 #pragma unroll
-                    for (int n = 0; n < NHIST; n++)
-                        asm volatile("prefetch.global.L2 [%0];" ::"l"(h + n * p.snap_plane));
+                for (int j = 0; j < QPT; j++) {
+                    const int w = quad[j].ix - p.snap_x1;
+                    if (quad[j].mine && dzr >= 0 && iz <= p.snap_z2 && dzr % p.snap_dz == 0 && w >= 0 && w < p.snx)
+#pragma unroll
+                        for (int n = 0; n < NHIST; n++)
+                            asm volatile("prefetch.global.L2 [%0];" ::"l"(row + w + n * p.snap_plane));
                 }
             }
         if (k) {
@@ -305,7 +338,13 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
         // ---- stress: vdiff2 + pml_diff2 + update_s2 + surf_mirror
         // (src/cpu/n_kernel_lib_PSV.cpp:100-205, 272-395).  A top free surface
         // and the rows it mirrors lie in the first band of tiles.
-        if (mask) {
+#pragma unroll
+        for (int j_ = 0; j_ < QPT; j_++) {
+            Quad &t = quad[j_];
+            if (!t.mask) continue;
+            const unsigned mask = t.mask;
+            const bool keep = t.keep;
+            const int ix = t.ix, o = o0 + 32 * j_, i = iz * p.pitch + ix;
             const Q4 cl = ldro4(p.c_lam + i), c2 = ldro4(p.c_l2m + i), cm = ldro4(p.c_muzx + i);
             const float *hz = sv + o - NS * RS, *hx = hz + HP;
             Q4 zz, xx, zx, xz;  // vz_z, vx_x, vz_x, vx_z
@@ -326,18 +365,18 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
                 xz = dvert<NS>(w, p.cz);
                 xx = dhorz<NS, 0>(h, p.cx);
             }
-            if (strip.z) {
-                cpml_quad(mz[MZ_VZ], all4(p.a_z[iz]), all4(p.b_z[iz]), all4(p.ki_z[iz]), zz, mask);
-                cpml_quad(mz[MZ_VX], all4(p.ah_z[iz]), all4(p.bh_z[iz]), all4(p.khi_z[iz]), xz, mask);
+            if (t.z) {
+                cpml_at<QPT>(t.mz[MZ_VZ], t.z + MZ_VZ * p.mz_plane, all4(p.a_z[iz]), all4(p.b_z[iz]), all4(p.ki_z[iz]), zz, mask);
+                cpml_at<QPT>(t.mz[MZ_VX], t.z + MZ_VX * p.mz_plane, all4(p.ah_z[iz]), all4(p.bh_z[iz]), all4(p.khi_z[iz]), xz, mask);
             }
-            if (strip.x) {
-                cpml_quad(mx[MX_VX], ldro4(p.a_x + ix), ldro4(p.b_x + ix), ldro4(p.ki_x + ix), xx, mask);
-                cpml_quad(mx[MX_VZ], ldro4(p.ah_x + ix), ldro4(p.bh_x + ix), ldro4(p.khi_x + ix), zx, mask);
+            if (t.x) {
+                cpml_at<QPT>(t.mx[MX_VX], t.x + MX_VX * p.mx_plane, ldro4(p.a_x + ix), ldro4(p.b_x + ix), ldro4(p.ki_x + ix), xx, mask);
+                cpml_at<QPT>(t.mx[MX_VZ], t.x + MX_VZ * p.mx_plane, ldro4(p.ah_x + ix), ldro4(p.bh_x + ix), ldro4(p.khi_x + ix), zx, mask);
             }
             Q4 szz = lds4(ss + o), szx = lds4(ss + HP + o), sxx = lds4(ss + 2 * HP + o);
             const bool image = p.st && iz == p.st, wz = !p.st || iz >= p.st;
             if (FWD && keep) {
-                float *r = kept + (F_SZZ - F_VZ) * KP + ko;
+                float *r = kept + (F_SZZ - F_VZ) * KP + ko0 + 32 * j_;
                 Q4 rzz = lds4(r), rzx = lds4(r + KP), rxx = lds4(r + 2 * KP);
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
@@ -370,7 +409,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
             }
             st4(ss + 2 * HP + o, sxx);
             if (p.st && iz > p.st && iz <= 2 * p.st - p.nz1) {
-                float *d = ss + (2 * p.st - iz - z0 + NS) * RS + HX + qc;
+                float *d = ss + (2 * p.st - iz - z0 + NS) * RS + HX + ix - x0;
 #pragma unroll
                 for (int j = 0; j < 4; j++)
                     if (mask >> j & 1) {
@@ -390,7 +429,13 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
         if (__syncthreads_or(failed)) break;
         // ---- velocity: sdiff2 + pml_diff2 + update_v2
         // (src/cpu/n_kernel_lib_PSV.cpp:207-270)
-        if (mask) {
+#pragma unroll
+        for (int j_ = 0; j_ < QPT; j_++) {
+            Quad &t = quad[j_];
+            if (!t.mask) continue;
+            const unsigned mask = t.mask;
+            const bool keep = t.keep;
+            const int ix = t.ix, o = o0 + 32 * j_, i = iz * p.pitch + ix;
             const float *azz = ss + o - NS * RS, *azx = azz + HP, *axx = azx + HP;
             Q4 vz = lds4(sv + o), vx = lds4(sv + HP + o);
             const Q4 crz = ldro4(p.c_rz + i), crx = ldro4(p.c_rx + i);
@@ -412,16 +457,16 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
             }
             row12(axx + NS * RS, lds4(axx + NS * RS), h);
             xx_x = dhorz<NS, 1>(h, p.cx);
-            if (strip.z) {
-                cpml_quad(mz[MZ_SZZ], all4(p.a_z[iz]), all4(p.b_z[iz]), all4(p.ki_z[iz]), zz_z, mask);
-                cpml_quad(mz[MZ_SZX], all4(p.ah_z[iz]), all4(p.bh_z[iz]), all4(p.khi_z[iz]), zx_z, mask);
+            if (t.z) {
+                cpml_at<QPT>(t.mz[MZ_SZZ], t.z + MZ_SZZ * p.mz_plane, all4(p.a_z[iz]), all4(p.b_z[iz]), all4(p.ki_z[iz]), zz_z, mask);
+                cpml_at<QPT>(t.mz[MZ_SZX], t.z + MZ_SZX * p.mz_plane, all4(p.ah_z[iz]), all4(p.bh_z[iz]), all4(p.khi_z[iz]), zx_z, mask);
             }
-            if (strip.x) {
-                cpml_quad(mx[MX_SXX], ldro4(p.a_x + ix), ldro4(p.b_x + ix), ldro4(p.ki_x + ix), xx_x, mask);
-                cpml_quad(mx[MX_SZX], ldro4(p.ah_x + ix), ldro4(p.bh_x + ix), ldro4(p.khi_x + ix), zx_x, mask);
+            if (t.x) {
+                cpml_at<QPT>(t.mx[MX_SXX], t.x + MX_SXX * p.mx_plane, ldro4(p.a_x + ix), ldro4(p.b_x + ix), ldro4(p.ki_x + ix), xx_x, mask);
+                cpml_at<QPT>(t.mx[MX_SZX], t.x + MX_SZX * p.mx_plane, ldro4(p.ah_x + ix), ldro4(p.bh_x + ix), ldro4(p.khi_x + ix), zx_x, mask);
             }
             Q4 rz = all4(0.f), rx = all4(0.f);
-            float *r = kept + ko;
+            float *r = kept + ko0 + 32 * j_;
             if (FWD && keep) {
                 rz = lds4(r);
                 rx = lds4(r + KP);
@@ -430,8 +475,8 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
             for (int j = 0; j < 4; j++) {
                 if (!(mask >> j & 1)) continue;
                 if constexpr (U) {
-                    uz.v[j] = fmaf(p.dt, vz.v[j], uz.v[j]);
-                    ux.v[j] = fmaf(p.dt, vx.v[j], ux.v[j]);
+                    t.uz.v[j] = fmaf(p.dt, vz.v[j], t.uz.v[j]);
+                    t.ux.v[j] = fmaf(p.dt, vx.v[j], t.ux.v[j]);
                 }
                 if (!FWD || !keep) {
                     vz.v[j] = fmaf(crz.v[j], zx_x.v[j] + zz_z.v[j], vz.v[j]);
@@ -440,7 +485,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
                     keep_sum(vz.v[j], rz.v[j], fmaf(crz.v[j], zx_x.v[j] + zz_z.v[j], rz.v[j]));
                     keep_sum(vx.v[j], rx.v[j], fmaf(crx.v[j], xx_x.v[j] + zx_z.v[j], rx.v[j]));
                 }
-                if constexpr (WE) we.v[j] += fmaf(vx.v[j], vx.v[j], vz.v[j] * vz.v[j]);
+                if constexpr (WE) t.we.v[j] += fmaf(vx.v[j], vx.v[j], vz.v[j] * vz.v[j]);
             }
             st4(sv + o, vz);
             st4(sv + HP + o, vx);
@@ -481,9 +526,14 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
         if (k + 1 < run.nsteps) send_rim(sv, false, 2 * k + 2);
         // ---- while the rims travel: snapshot store (its velocities are the
         // injected ones) or imaging (src/cpu/n_kernel_lib_PSV.cpp:398-484)
-        if (slot >= 0 && mine)
-            snapshot_quad<MODE>(p, bz, iz, ix, slot, lds4(ss + o), lds4(ss + HP + o), lds4(ss + 2 * HP + o),
-                                lds4(sv + o), lds4(sv + HP + o), uz, ux);
+        if (slot >= 0)
+#pragma unroll
+            for (int j = 0; j < QPT; j++) {
+                const int o = o0 + 32 * j;
+                if (quad[j].mine)
+                    snapshot_quad<MODE>(p, bz, iz, quad[j].ix, slot, lds4(ss + o), lds4(ss + HP + o),
+                                        lds4(ss + 2 * HP + o), lds4(sv + o), lds4(sv + HP + o), quad[j].uz, quad[j].ux);
+            }
         // ---- urec2 (src/cpu/n_kernel_lib_PSV.cpp:533-576)
         if (recorder && e.r0 < e.r1) {
             const long long row = (long long)it * q.nrec;
@@ -504,94 +554,112 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
     }
     if (failed) atomicExch(p.err, 1);
     // ---- back to the field block
-    if (mine) {
 #pragma unroll
-        for (int k = 0; k < 5; k++) st4(f + (F_VZ + k) * p.plane, lds4(sm + k * HP + o));
-        if (keep)
+    for (int j = 0; j < QPT; j++) {
+        const Quad &t = quad[j];
+        const int o = o0 + 32 * j, ko = ko0 + 32 * j, i = iz * p.pitch + t.ix;
+        if (t.mine) {
 #pragma unroll
-            for (int k = 0; k < 5; k++) st4(fk + (F_VZ + k) * p.plane, lds4(kept + k * KP + ko));
-        if constexpr (WE) st4(f + (FWD ? F_WE : F_WEA) * p.plane, we);
-        if constexpr (U) {
-            st4(f + F_UZ * p.plane, uz);
-            st4(f + F_UX * p.plane, ux);
+            for (int k = 0; k < 5; k++) st4(fs + i + (F_VZ + k) * p.plane, lds4(sm + k * HP + o));
+            if (t.keep)
+#pragma unroll
+                for (int k = 0; k < 5; k++) st4(fk + i + (F_VZ + k) * p.plane, lds4(kept + k * KP + ko));
+            if constexpr (WE) st4(fs + i + (FWD ? F_WE : F_WEA) * p.plane, t.we);
+            if constexpr (U) {
+                st4(fs + i + F_UZ * p.plane, t.uz);
+                st4(fs + i + F_UX * p.plane, t.ux);
+            }
         }
+        if (QPT == 1 && t.z)
+#pragma unroll
+            for (int k = 0; k < 4; k++) st4(t.z + k * p.mz_plane, t.mz[k]);
+        if (QPT == 1 && t.x)
+#pragma unroll
+            for (int k = 0; k < 4; k++) st4(t.x + k * p.mx_plane, t.mx[k]);
     }
-    if (strip.z)
-#pragma unroll
-        for (int k = 0; k < 4; k++) st4(strip.z + k * p.mz_plane, mz[k]);
-    if (strip.x)
-#pragma unroll
-        for (int k = 0; k < 4; k++) st4(strip.x + k * p.mx_plane, mx[k]);
 }
 
-template <int NS, int MODE>
+template <int NS, int QPT, int MODE>
 cudaError_t resident_m(const StepParams<float> &p, const SrcRecParams<float> &q, const ResidentRun &g, int nbatch,
                        cudaStream_t st)
 {
-    auto kernel = k_resident<NS, MODE>;
+    constexpr int RW = 32 * QPT;
+    auto kernel = k_resident<NS, QPT, MODE>;
     static const cudaError_t opt_in = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           resident_smem(NS, MAX_THREADS / 8));
+                                                           resident_smem(NS, RW, MAX_THREADS / 8));
     if (opt_in != cudaSuccess) return opt_in;
     const int ctas = g.ntx * g.ntz * nbatch;
-    cudaError_t e = cudaMemsetAsync(g.inbox, 0, (size_t)ctas * 2 * rim_cells(NS, g.tz) * sizeof(ulonglong2), st);
+    cudaError_t e = cudaMemsetAsync(g.inbox, 0, (size_t)ctas * 2 * rim_cells(NS, RW, g.tz) * sizeof(ulonglong2), st);
     if (e != cudaSuccess) return e;
     StepParams<float> a = p;
     SrcRecParams<float> s = q;
     ResidentRun r = g;
     void *args[] = {&a, &s, &r};
-    return cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(resident_threads(NS, g.tz)), args,
-                                       (size_t)resident_smem(NS, g.tz), st);
+    return cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(resident_threads(NS, RW, g.tz)), args,
+                                       (size_t)resident_smem(NS, RW, g.tz), st);
 }
 
-template <int NS>
-cudaError_t resident_n(const StepParams<float> &p, const SrcRecParams<float> &q, const ResidentRun &g, int mode,
+template <int NS, int QPT>
+cudaError_t resident_q(const StepParams<float> &p, const SrcRecParams<float> &q, const ResidentRun &g, int mode,
                        int nbatch, cudaStream_t st)
 {
     switch (mode) {
-    case MODE_FWD: return resident_m<NS, MODE_FWD>(p, q, g, nbatch, st);
-    case MODE_FWD_NOWE: return resident_m<NS, MODE_FWD_NOWE>(p, q, g, nbatch, st);
-    case MODE_FWD_U: return resident_m<NS, MODE_FWD_U>(p, q, g, nbatch, st);
-    case MODE_ADJ: return resident_m<NS, MODE_ADJ>(p, q, g, nbatch, st);
+    case MODE_FWD: return resident_m<NS, QPT, MODE_FWD>(p, q, g, nbatch, st);
+    case MODE_FWD_NOWE: return resident_m<NS, QPT, MODE_FWD_NOWE>(p, q, g, nbatch, st);
+    case MODE_FWD_U: return resident_m<NS, QPT, MODE_FWD_U>(p, q, g, nbatch, st);
+    case MODE_ADJ: return resident_m<NS, QPT, MODE_ADJ>(p, q, g, nbatch, st);
     default: return cudaErrorInvalidValue;
     }
 }
 
-}  // namespace
-
-// Tile rows that give every CTA of a batch a place on `nsm` SMs at once: the
-// smallest from 8 (the mirrored rows of a top surface must fit) that needs one
-// CTA per SM, else the smallest that needs as many as fit; 0 if none does, or
-// with other surfaces, whose mirrored cells cross tiles.  512 threads of 128
-// registers fill an SM.
-int resident_rows(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm)
+template <int NS>
+cudaError_t resident_n(const StepParams<float> &p, const SrcRecParams<float> &q, const ResidentRun &g, int mode, int rw,
+                       int nbatch, cudaStream_t st)
 {
-    if (ns < 1 || ns > HX || sb || sl || sr) return 0;
-    const int ntx = (nx + RW - 1) / RW;
-    for (int most : {1, 4})
-        for (int tz = 8; tz <= MAX_THREADS / 8; tz++) {
-            if (st && 2 * st - nz1 >= tz) continue;
-            const long long ctas = (long long)ntx * ((nz + tz - 1) / tz) * nbatch;
-            const int per = std::min({most, MAX_THREADS / resident_threads(ns, tz),
-                                      227 * 1024 / (resident_smem(ns, tz) + 1024)});
-            if (ctas <= (long long)nsm * per) return tz;
-        }
-    return 0;
+    return rw == 32 ? resident_q<NS, 1>(p, q, g, mode, nbatch, st) : resident_q<NS, 2>(p, q, g, mode, nbatch, st);
 }
 
-size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, int tz)
+}  // namespace
+
+// Tiles that give every CTA of a batch a place on `nsm` SMs at once: 32
+// columns (one quad a thread) if the batch then fits, else 64 (two); the
+// fewest rows from 8 (the mirrored rows of a top surface must fit) that need
+// one CTA per SM, else the fewest with which as many as fit are enough.  tz =
+// 0 if nothing is, or with other surfaces, whose mirrored cells cross tiles.
+// 512 threads of 128 registers fill an SM.
+ResidentTile resident_tile(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm)
 {
-    return (size_t)((nx + RW - 1) / RW) * ((nz + tz - 1) / tz) * nbatch * 2 * rim_cells(ns, tz) * sizeof(ulonglong2);
+    if (ns < 1 || ns > HX || sb || sl || sr) return {0, 0};
+    for (int rw : {32, 64}) {
+        const int ntx = (nx + rw - 1) / rw;
+        for (int most : {1, 4})
+            for (int tz = 8; tz <= MAX_THREADS / 8; tz++) {
+                if (st && 2 * st - nz1 >= tz) continue;
+                const long long ctas = (long long)ntx * ((nz + tz - 1) / tz) * nbatch;
+                const int per = std::min({most, MAX_THREADS / resident_threads(ns, rw, tz),
+                                          227 * 1024 / (resident_smem(ns, rw, tz) + 1024)});
+                if (ctas <= (long long)nsm * per) return {rw, tz};
+            }
+    }
+    return {0, 0};
+}
+
+size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, const ResidentTile &t)
+{
+    return (size_t)((nx + t.rw - 1) / t.rw) * ((nz + t.tz - 1) / t.tz) * nbatch * 2 * rim_cells(ns, t.rw, t.tz) *
+           sizeof(ulonglong2);
 }
 
 cudaError_t launch_resident(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopRun &run, int ns,
-                            int mode, int tz, int nbatch, cudaStream_t st)
+                            int mode, const ResidentTile &t, int nbatch, cudaStream_t st)
 {
-    const ResidentRun g{run, tz, (p.nx + RW - 1) / RW, (p.nz + tz - 1) / tz, reinterpret_cast<ulonglong2 *>(run.sync)};
+    const ResidentRun g{run, t.tz, (p.nx + t.rw - 1) / t.rw, (p.nz + t.tz - 1) / t.tz,
+                        reinterpret_cast<ulonglong2 *>(run.sync)};
     switch (ns) {
-    case 1: return resident_n<1>(p, q, g, mode, nbatch, st);
-    case 2: return resident_n<2>(p, q, g, mode, nbatch, st);
-    case 3: return resident_n<3>(p, q, g, mode, nbatch, st);
-    case 4: return resident_n<4>(p, q, g, mode, nbatch, st);
+    case 1: return resident_n<1>(p, q, g, mode, t.rw, nbatch, st);
+    case 2: return resident_n<2>(p, q, g, mode, t.rw, nbatch, st);
+    case 3: return resident_n<3>(p, q, g, mode, t.rw, nbatch, st);
+    case 4: return resident_n<4>(p, q, g, mode, t.rw, nbatch, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -55,7 +55,7 @@ typedef enum {
 #define PSV_KERNELS_TMA 2       /* tiles staged in shared memory by TMA tensor copies; up to
                                    hundreds of time steps per launch with no free surface or a
                                    top one whose mirrored rows fit the first tile; with
-                                   rows_per_thread 8 and a batch that fits the GPU's SMs at 2048
+                                   rows_per_thread 8 and a batch that fits the GPU's SMs at 4096
                                    points each, wavefields stay on chip between the steps (FP32) */
 #define PSV_KERNELS_VEC4 3      /* four columns per thread, 128-bit loads and stores (FP32) */
 #define PSV_KERNELS_FUSED 4     /* one launch per time step: stress of a tile and its halo,

@@ -93,7 +93,7 @@ def test_two_plans_at_once(gpu):
 
 def test_the_shape_a_plan_starts_with(gpu):
     # 500 000 points of a batch and a surface the loop handles
-    for nz, nx, nshot, precision, isurf, family in ((501, 1001, 1, 32, None, "tma"), (301, 601, 2, 32, None, "direct"),
+    for nz, nx, nshot, precision, isurf, family in ((501, 1001, 1, 32, None, "tma"), (301, 601, 2, 32, None, "tma"),
                                                     (301, 601, 4, 32, None, "tma"), (501, 1001, 1, 64, None, "direct"),
                                                     (501, 1001, 1, 32, (40, 0, 0, 0), "direct")):
         sv, _, _ = helpers.case(nz=nz, nx=nx, nshot=nshot, nt=4, surf_offset=0)

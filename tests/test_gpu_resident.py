@@ -29,7 +29,9 @@ def _surface(nz, nx, order, nshot, nt=150, nrec=12, rec_spacing=4, **kw):
 @pytest.mark.parametrize("order,nz,nx,nshot", [
     (2, 16, 31, 1), (4, 31, 33, 2), (6, 47, 131, 2), (8, 41, 129, 2), (4, 64, 128, 1), (8, 97, 190, 2),
     (4, 301, 601, 1),   # tiles of 38 rows
-    (2, 330, 288, 3)])  # four CTAs on an SM
+    (2, 330, 288, 3),   # four CTAs on an SM
+    (8, 211, 333, 4),   # two quads a thread
+    (6, 380, 701, 2)])  # ... in tiles of 64 rows
 def test_ragged_grids_with_a_surface(gpu, order, nz, nx, nshot):
     _both(*_surface(nz, nx, order, nshot, snap_dt=2), 8)
 
