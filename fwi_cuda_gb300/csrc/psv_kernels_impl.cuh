@@ -392,15 +392,16 @@ __device__ __forceinline__ void srcrec_apply(const StepParams<T> &p, const SrcRe
     if (recs) {
         double *rz = q.rtf_z + shot * q.rtf_shot_stride;
         double *rx = q.rtf_x + shot * q.rtf_shot_stride;
-        const double ru = q.rec_unscale[shot];
+        // one factor: FP64 divides run at a 64th of the FP32 rate
+        const double ru = q.dt_d * q.inv_dzdx * q.rec_unscale[shot];
         const long long row = (long long)it * q.nrec;
         for (int k = e.r0 + tid; k < e.r1; k += nth) {
             const int rr = q.t_rec_r[k];
             const int pos = q.rec_pos[rr];
             const double pz = it ? rz[row - q.nrec + rr] : 0.0;
             const double px = it ? rx[row - q.nrec + rr] : 0.0;
-            rz[row + rr] = pz + ((q.dt_d * (double)vz[pos]) / q.dzdx) * ru;
-            rx[row + rr] = px + ((q.dt_d * (double)vx[pos]) / q.dzdx) * ru;
+            rz[row + rr] = fma(ru, (double)vz[pos], pz);
+            rx[row + rr] = fma(ru, (double)vx[pos], px);
         }
     }
     if (slot >= 0 && q.src_kind == 0 && MODE != MODE_ADJ) {  // snapshot holds post-injection v

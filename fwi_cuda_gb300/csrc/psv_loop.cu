@@ -489,15 +489,17 @@ __device__ __forceinline__ void srcrec_warp(const StepParams<float> &p, const Sr
     if (e.r0 < e.r1) {
         double *rz = q.rtf_z + shot * q.rtf_shot_stride;
         double *rx = q.rtf_x + shot * q.rtf_shot_stride;
-        const double ru = q.rec_unscale[shot];
+        // one factor: an FP64 divide a sample holds up the tile's publication
+        // (FP64 runs at a 64th of the FP32 rate)
+        const double ru = q.dt_d * q.inv_dzdx * q.rec_unscale[shot];
         const long long row = (long long)T.it * q.nrec;
         for (int k = e.r0 + lane; k < e.r1; k += 32) {
             const int rr = q.t_rec_r[k];
             const int i = local(q.rec_pos[rr]);
             const double pz = T.it ? __ldcg(rz + row - q.nrec + rr) : 0.0;
             const double px = T.it ? __ldcg(rx + row - q.nrec + rr) : 0.0;
-            rz[row + rr] = pz + ((q.dt_d * (double)vz[i]) / q.dzdx) * ru;
-            rx[row + rr] = px + ((q.dt_d * (double)vx[i]) / q.dzdx) * ru;
+            rz[row + rr] = fma(ru, (double)vz[i], pz);
+            rx[row + rr] = fma(ru, (double)vx[i], px);
         }
     }
     if (MODE != MODE_ADJ && T.slot >= 0 && q.src_kind == 0) {
