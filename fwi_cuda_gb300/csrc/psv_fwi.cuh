@@ -57,6 +57,10 @@ cudaError_t launch_adjoint_scale(const double *res_z, const double *res_x, long 
                                  double *ascale, cudaStream_t st);
 
 // Deterministic FP64 sums: partial sums by a fixed grid, then one block.
+// Smallest positive lam + mu, largest lam + 2 mu and smallest rho above 1e-4 of
+// n cells (infinities where there is none): kRedBlocks values of each in `out`.
+cudaError_t launch_model_extremes(const double *lam, const double *mu, const double *rho, long long n, double *out,
+                                  cudaStream_t st);
 cudaError_t launch_model_sums(const double *lam, const double *mu, const double *rho, int nz,
                               int nx, double *partial, double *out3, cudaStream_t st);
 // Blocks of the first stage of the deterministic reductions: launch_adjsrc

@@ -131,6 +131,51 @@ __global__ void __launch_bounds__(RED_THREADS) k_final_sum(const double *partial
     if (threadIdx.x == 0) out[blockIdx.x] = s * scale;
 }
 
+// The extremes the range scales need, where the model is: compares only, in
+// any order.  24 bytes a cell, 7 us on 1001 x 2001; the same on the host with
+// a divide a cell took 3.9 ms.
+__global__ void __launch_bounds__(RED_THREADS) k_model_extremes(const double *lam, const double *mu,
+                                                                const double *rho, long long n, double *out)
+{
+    __shared__ double sh[3][RED_THREADS / 32];
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    double lo = inf, hi = -inf, rl = inf;
+    for (long long k = (long long)blockIdx.x * RED_THREADS + threadIdx.x; k < n;
+         k += (long long)RED_BLOCKS * RED_THREADS) {
+        const double l = lam[k], m = mu[k], r = rho[k], a = l + m, b = l + 2.0 * m;
+        if (a > 0 && a < lo) lo = a;
+        if (b > hi) hi = b;
+        if (r > 1e-4 && r < rl) rl = r;
+    }
+    for (int o = 16; o; o >>= 1) {
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        rl = fmin(rl, __shfl_xor_sync(0xffffffffu, rl, o));
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][w] = lo;
+        sh[1][w] = hi;
+        sh[2][w] = rl;
+    }
+    __syncthreads();
+    if (threadIdx.x) return;
+    for (int k = 1; k < RED_THREADS / 32; k++) {
+        lo = fmin(lo, sh[0][k]);
+        hi = fmax(hi, sh[1][k]);
+        rl = fmin(rl, sh[2][k]);
+    }
+    out[blockIdx.x] = lo;
+    out[RED_BLOCKS + blockIdx.x] = hi;
+    out[2 * RED_BLOCKS + blockIdx.x] = rl;
+}
+cudaError_t launch_model_extremes(const double *lam, const double *mu, const double *rho, long long n, double *out,
+                                  cudaStream_t st)
+{
+    k_model_extremes<<<RED_BLOCKS, RED_THREADS, 0, st>>>(lam, mu, rho, n, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_model_sums(const double *lam, const double *mu, const double *rho, int nz,
                               int nx, double *partial, double *out3, cudaStream_t st)
 {

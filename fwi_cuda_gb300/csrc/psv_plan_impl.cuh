@@ -1197,24 +1197,33 @@ public:
 
     static double pow2_near(double x) { return (x > 0 && std::isfinite(x)) ? std::exp2(-std::rint(std::log2(x))) : 1.0; }
 
-    // Range scales from a host model: forward source gain (exact powers of two).
-    void model_scales(const double *l, const double *m, double inv_rho_max)
+    // Extremes of the model on the device (launch_model_extremes).
+    int model_extremes(double *lm_min, double *l2m_max, double *rho_min)
+    {
+        double h[3 * kRedBlocks];
+        PSV_CU(launch_model_extremes(lam(), mu(), rho(), (long long)sv.g.nz * sv.g.nx, partial(), st));
+        PSV_CU(cudaMemcpyAsync(h, partial(), sizeof(h), cudaMemcpyDeviceToHost, st));
+        PSV_CU(cudaStreamSynchronize(st));
+        *lm_min = *std::min_element(h, h + kRedBlocks);
+        *l2m_max = *std::max_element(h + kRedBlocks, h + 2 * kRedBlocks);
+        *rho_min = *std::min_element(h + 2 * kRedBlocks, h + 3 * kRedBlocks);
+        return PSV_OK;
+    }
+
+    // Range scales of a model: forward source gain (exact powers of two).  Both
+    // maxima are monotone in an extreme of the model, so no cell costs a divide.
+    void model_scales(double lm_min, double l2m_max, double inv_rho_max)
     {
         const psv_grid &g = sv.g;
-        const size_t n = (size_t)g.nz * g.nx;
         inj = g.dt / (g.dz * g.dx) * inv_rho_max;
         double amax = 0.0;
         for (double v : sv.stf_z) amax = std::max(amax, std::fabs(v));
         for (double v : sv.stf_x) amax = std::max(amax, std::fabs(v));
         const double sf = pow2_near(sv.s.stf_type == 0 ? amax * inj : amax);
         // imaging factor: g1 * (dt (lam + 2 mu) / dz)^2 ~ 1 with unit-scaled fields
-        double g1max = 0.0, cmax = 0.0;
         const double kimg = (double)g.snap_dt * g.dt;
-        for (size_t k = 0; k < n; k++) {
-            const double lm = l[k] + m[k];
-            if (lm > 0) g1max = std::max(g1max, kimg * 0.25 / (lm * lm));
-            cmax = std::max(cmax, g.dt * (l[k] + 2.0 * m[k]) / std::min(g.dz, g.dx));
-        }
+        const double g1max = std::max(0.0, kimg * 0.25 / (lm_min * lm_min));
+        const double cmax = std::max(0.0, g.dt * l2m_max / std::min(g.dz, g.dx));
         gscale = pow2_near(g1max * cmax * cmax);
         std::vector<double> h((size_t)2 * sv.s.nshot);
         for (int s_ = 0; s_ < sv.s.nshot; s_++) { h[s_] = sf; h[sv.s.nshot + s_] = 1.0 / sf; }
@@ -1224,13 +1233,12 @@ public:
     int set_model(const double *l, const double *m, const double *r) override
     {
         const size_t n = (size_t)sv.g.nz * sv.g.nx;
-        double rmin = 0.0;
-        for (size_t k = 0; k < n; k++)
-            if (r[k] > 1e-4 && (rmin == 0.0 || r[k] < rmin)) rmin = r[k];
-        model_scales(l, m, rmin > 0 ? 1.0 / rmin : 1.0);
         PSV_CU(cudaMemcpyAsync(lam(), l, n * 8, cudaMemcpyHostToDevice, st));
         PSV_CU(cudaMemcpyAsync(mu(), m, n * 8, cudaMemcpyHostToDevice, st));
         PSV_CU(cudaMemcpyAsync(rho(), r, n * 8, cudaMemcpyHostToDevice, st));
+        double lm, l2m, rmin;
+        PSV_TRY(model_extremes(&lm, &l2m, &rmin));
+        model_scales(lm, l2m, std::isfinite(rmin) ? 1.0 / rmin : 1.0);
         PSV_TRY(coefficients(true, false));
         have_model = true;
         return PSV_OK;
@@ -2134,7 +2142,9 @@ public:
         PSV_CU(cudaMemcpyAsync(avg(2), rxp, n * 8, cudaMemcpyHostToDevice, st));
         double rzmax = 0.0;
         for (size_t k = 0; k < n; k++) rzmax = std::max(rzmax, std::max(std::fabs(rzp[k]), std::fabs(rxp[k])));
-        model_scales(l, m, rzmax > 0 ? rzmax : 1.0);
+        double lm, l2m, rmin;
+        PSV_TRY(model_extremes(&lm, &l2m, &rmin));  // (no density here: rmin unused)
+        model_scales(lm, l2m, rzmax > 0 ? rzmax : 1.0);
         double sc = 1.0;  // amplitude scale of this call's wavefields
         PSV_CU(cudaMemcpy(&sc, fscale(), 8, cudaMemcpyDeviceToHost));
         if (grad_) {  // adjoint sources are the caller's: same rule as the forward gain
