@@ -392,16 +392,21 @@ __device__ __forceinline__ void srcrec_apply(const StepParams<T> &p, const SrcRe
     if (recs) {
         double *rz = q.rtf_z + shot * q.rtf_shot_stride;
         double *rx = q.rtf_x + shot * q.rtf_shot_stride;
-        // one factor: FP64 divides run at a 64th of the FP32 rate
-        const double ru = q.dt_d * q.inv_dzdx * q.rec_unscale[shot];
+        // FP32 plans: one factor; FP64 divides run at a 64th of the FP32 rate.
+        // FP64 plans round every operation as the reference does.
+        const double us = q.rec_unscale[shot], ru = q.dt_d * q.inv_dzdx * us;
+        auto sample = [&](double v, double before) {
+            if constexpr (sizeof(T) == 4) return fma(ru, v, before);
+            else return before + ((q.dt_d * v) / q.dzdx) * us;
+        };
         const long long row = (long long)it * q.nrec;
         for (int k = e.r0 + tid; k < e.r1; k += nth) {
             const int rr = q.t_rec_r[k];
             const int pos = q.rec_pos[rr];
             const double pz = it ? rz[row - q.nrec + rr] : 0.0;
             const double px = it ? rx[row - q.nrec + rr] : 0.0;
-            rz[row + rr] = fma(ru, (double)vz[pos], pz);
-            rx[row + rr] = fma(ru, (double)vx[pos], px);
+            rz[row + rr] = sample((double)vz[pos], pz);
+            rx[row + rr] = sample((double)vx[pos], px);
         }
     }
     if (slot >= 0 && q.src_kind == 0 && MODE != MODE_ADJ) {  // snapshot holds post-injection v
