@@ -5,6 +5,7 @@
 #pragma once
 
 #include "psv_kernels_impl.cuh"
+#include "psv_surface.hpp"
 
 namespace psv {
 namespace {

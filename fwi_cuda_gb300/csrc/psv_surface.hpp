@@ -1,0 +1,27 @@
+// psv_surface.hpp -- the rows beside a top free surface (host and device).
+#pragma once
+
+#ifdef __CUDACC__
+#define PSV_HD __host__ __device__ __forceinline__
+#else
+#define PSV_HD inline
+#endif
+
+namespace psv {
+
+// What interior row iz has to do with a top free surface on row st (0: none)
+// above which the interior starts at nz1 (surf_mirror,
+// src/cpu/n_kernel_lib_PSV.cpp:272-395).  Rows [nz1, st) take szz and szx from
+// the rows they mirror: their own threads leave both alone, so that every cell
+// has one writer and, in a phase of the update, no other reader.
+struct SurfaceRow {
+    bool own;    // szz and szx are this row's own, not mirrored into it
+    bool image;  // the surface row itself
+    int mirror;  // the row this row's szz and szx are mirrored into, or -1
+};
+PSV_HD SurfaceRow surface_row(int iz, int st, int nz1)
+{
+    return {!st || iz >= st, st && iz == st, st && iz > st && iz <= 2 * st - nz1 ? 2 * st - iz : -1};
+}
+
+}  // namespace psv
