@@ -487,20 +487,23 @@ public:
 
     // Whether the plan may choose its kernels.
     bool any_kernels() const { return opt.kernel_family == 0 && opt.rows_per_thread == 0; }
-    // The shape of a plan nobody autotunes (modelling).  The resident kernel
-    // where the batch fits it (a block shape given is the direct family's):
-    // 2.9 us a step against 9.0 on 101 x 201, 3.6 against 11 on 301 x 601, 6.9
-    // against 12 on 281 x 561, 2 shots.  Beyond, from 500 000 points in a batch,
-    // the looped TMA tiles beat the direct kernels: 12.7 against 14.1 us a step
-    // at 0.54 M points (301 x 601, 3 shots, order 4), 16.5 against 25.9 at 1.4 M,
-    // 21 against 40 at 2.0 M (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
+    // The shape of a plan nobody autotunes (modelling).  A block shape or a chain
+    // count given (one chain too) is the direct family's, and it runs; its blocks
+    // are 32 columns wide, so another block_x gives none.  Else the resident
+    // kernel where the batch fits it: 2.9 us a step against 9.0 on
+    // 101 x 201, 3.6 against 11 on 301 x 601, 6.9 against 12 on 281 x 561, 2
+    // shots.  Beyond, from 500 000 points in a batch, the looped TMA tiles beat
+    // the direct kernels: 12.7 against 14.1 us a step at 0.54 M points (301 x 601,
+    // 3 shots, order 4), 16.5 against 25.9 at 1.4 M, 21 against 40 at 2.0 M
+    // (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
     int start_shape(int *r) const
     {
-        if (rt.tz && !beside && opt.chains == 0) {
+        const bool given = (opt.block_y > 0 && (opt.block_x <= 0 || opt.block_x == 32)) || opt.chains != 0;
+        if (rt.tz && !beside && !given) {
             *r = 8;
             return PSV_KERNELS_TMA;
         }
-        if (sizeof(T) == 4 && opt.block_y <= 0 && (double)sv.g.nz * sv.g.nx * B >= 500e3 &&
+        if (sizeof(T) == 4 && !given && (double)sv.g.nz * sv.g.nx * B >= 500e3 &&
             loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
             *r = 4;
             return PSV_KERNELS_TMA;

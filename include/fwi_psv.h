@@ -156,7 +156,8 @@ typedef struct psv_options {
                                    1, 2, 4; FUSED family: tile rows 16 or 32; MARCH family:
                                    rows each CTA marches, 32, 64 or 128; 0 = default */
     int kernel_family;          /* time-step kernels: 0 = any (the autotuner chooses; before
-                                   and without it, by the batch's grid points),
+                                   and without it, by the batch's grid points, or the direct
+                                   family where block_y (block_x 0 or 32) or chains is given),
                                    PSV_KERNELS_DIRECT, _TMA, _VEC4, _FUSED or _MARCH (the
                                    last four FP32 only; FUSED needs no free surface but a top
                                    one, MARCH none or a top one on the first interior row) */
