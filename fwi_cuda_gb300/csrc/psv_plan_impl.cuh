@@ -490,12 +490,18 @@ public:
     // The shape of a plan nobody autotunes (modelling).  A block shape or a chain
     // count given (one chain too) is the direct family's, and it runs; its blocks
     // are 32 columns wide, so another block_x gives none.  Else the resident
-    // kernel where the batch fits it: 2.9 us a step against 9.0 on
-    // 101 x 201, 3.6 against 11 on 301 x 601, 6.9 against 12 on 281 x 561, 2
-    // shots.  Beyond, from 500 000 points in a batch, the looped TMA tiles beat
-    // the direct kernels: 12.7 against 14.1 us a step at 0.54 M points (301 x 601,
-    // 3 shots, order 4), 16.5 against 25.9 at 1.4 M, 21 against 40 at 2.0 M
-    // (1001 x 2001, order 8), and 12.0 against 11.9 at 0.36 M.
+    // kernel where the batch fits it: 2.9 us a step against 9.0 on 101 x 201, 3.6
+    // against 11 on 301 x 601, 6.9 against 12 on 281 x 561, 2 shots.  Beyond, the
+    // looped TMA tiles, whose velocity tiles follow the stress tiles a few bands of
+    // 16 rows behind, on batches and grids with enough of both (direct / tile list,
+    // modelling, orders 4 and 8, nx from 72 to 4000; above 1: the list is faster):
+    //   bands      0.5 M points  0.75 M      1.25 M      2.5 M        5 and 10 M
+    //   2          0.84 - 0.98   0.96 - 1.1  1.1         0.93 - 1.0   0.8 - 0.9
+    //   3, 4       0.59 - 0.73   0.66 - 0.9  0.80 - 1.1  0.94 - 1.07  1.0 - 1.4
+    //   5          0.83 - 1.03   0.95 - 1.2  1.1 - 1.3   1.25 - 1.3   1.2 - 1.5
+    //   7          0.92 - 1.2    1.03 - 1.3  1.2 - 1.4   1.2 - 1.3
+    //   9 and 13   0.96 - 1.3    1.1 - 1.4   1.2 - 1.5   1.2 - 1.6
+    // (1001 x 2001, order 8, one shot: 40 against 21 us a step).
     int start_shape(int *r) const
     {
         const bool given = (opt.block_y > 0 && (opt.block_x <= 0 || opt.block_x == 32)) || opt.chains != 0;
@@ -503,7 +509,10 @@ public:
             *r = 8;
             return PSV_KERNELS_TMA;
         }
-        if (sizeof(T) == 4 && !given && (double)sv.g.nz * sv.g.nx * B >= 500e3 &&
+        const int bands = (sv.g.nz + 15) / 16;
+        const double points = (double)sv.g.nz * sv.g.nx * B;
+        const double least = bands >= 9 ? 0.5e6 : bands >= 5 ? 1e6 : 4e6;
+        if (sizeof(T) == 4 && !given && bands >= 3 && points >= least &&
             loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
             *r = 4;
             return PSV_KERNELS_TMA;
