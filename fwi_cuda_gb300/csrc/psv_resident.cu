@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
 
     // A mirrored row's szz and szx are other threads' to write while its own
     // reads stresses: it reads v in their place, and writes neither.  (One
-    // offset for the launch; the rest of surface_row is spelled out below:
-    // 2.75 us a step on 101 x 201, 2.83 with its flags held through a step.)
-    const int own0 = surface_row(iz, p.st, p.nz1).own ? o0 : o0 - 2 * HP;
+    // offset for the launch: 2.75 us a step on 101 x 201, 2.83 with loads under
+    // a predicate in each step.)
+    const int own0 = surface_own(iz, p.st) ? o0 : o0 - 2 * HP;
     bool failed = false;
     for (int k = 0; k < run.nsteps; k++) {
         const int it = run.it0 + k * run.dit, rel = it / run.sdt;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
                 cpml_at<QPT>(t.mx[MX_VX], t.x + MX_VX * p.mx_plane, ldro4(p.a_x + ix), ldro4(p.b_x + ix), ldro4(p.ki_x + ix), xx, mask);
                 cpml_at<QPT>(t.mx[MX_VZ], t.x + MX_VZ * p.mx_plane, ldro4(p.ah_x + ix), ldro4(p.bh_x + ix), ldro4(p.khi_x + ix), zx, mask);
             }
-            const bool image = p.st && iz == p.st;
+            const bool image = surface_image(iz, p.st);
             const float *own = ss + own0 + 32 * j_;
             Q4 szz = lds4(own), szx = lds4(own + HP), sxx = lds4(ss + 2 * HP + o);
             if (FWD && keep) {
@@ -409,12 +409,12 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
                     sxx.v[j] = p.fs_top[ix + j] * xx.v[j];
                 }
             }
-            if (!p.st || iz >= p.st) {  // szz, szx are this row's own
+            if (surface_own(iz, p.st)) {
                 st4(ss + o, szz);
                 st4(ss + HP + o, szx);
             }
             st4(ss + 2 * HP + o, sxx);
-            if (p.st && iz > p.st && iz <= 2 * p.st - p.nz1) {
+            if (surface_mirrors(iz, p.st, p.nz1)) {
                 float *d = ss + (2 * p.st - iz - z0 + NS) * RS + HX + ix - x0;
 #pragma unroll
                 for (int j = 0; j < 4; j++)

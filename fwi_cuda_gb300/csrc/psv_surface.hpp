@@ -14,14 +14,11 @@ namespace psv {
 // src/cpu/n_kernel_lib_PSV.cpp:272-395).  Rows [nz1, st) take szz and szx from
 // the rows they mirror: their own threads leave both alone, so that every cell
 // has one writer and, in a phase of the update, no other reader.
-struct SurfaceRow {
-    bool own;    // szz and szx are this row's own, not mirrored into it
-    bool image;  // the surface row itself
-    int mirror;  // the row this row's szz and szx are mirrored into, or -1
-};
-PSV_HD SurfaceRow surface_row(int iz, int st, int nz1)
+PSV_HD bool surface_own(int iz, int st) { return !st || iz >= st; }     // szz, szx are the row's own
+PSV_HD bool surface_image(int iz, int st) { return st && iz == st; }    // the surface row itself
+PSV_HD bool surface_mirrors(int iz, int st, int nz1)                    // mirrored into row 2 st - iz
 {
-    return {!st || iz >= st, st && iz == st, st && iz > st && iz <= 2 * st - nz1 ? 2 * st - iz : -1};
+    return st && iz > st && iz <= 2 * st - nz1;
 }
 
 }  // namespace psv

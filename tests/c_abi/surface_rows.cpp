@@ -14,11 +14,10 @@ int main()
                 if (st && st < nz1) continue;
                 std::vector<int> own(nz, 0), written(nz, 0);
                 for (int iz = nz1; iz < nz - nz1; iz++) {
-                    const psv::SurfaceRow r = psv::surface_row(iz, st, nz1);
-                    own[iz] = r.own;  // reads and writes its own cells
-                    written[iz] += r.own;
-                    if (r.mirror >= 0) written[r.mirror]++;
-                    if (r.image != (st && iz == st)) return printf("image row %d, surface %d\n", iz, st), 1;
+                    own[iz] = psv::surface_own(iz, st);  // reads and writes its own cells
+                    written[iz] += own[iz];
+                    if (psv::surface_mirrors(iz, st, nz1)) written[2 * st - iz]++;
+                    if (psv::surface_image(iz, st) != (st && iz == st)) return printf("image row %d, surface %d\n", iz, st), 1;
                 }
                 for (int iz = nz1; iz < nz - nz1; iz++, n++) {
                     const bool mirrored = st && iz < st;
