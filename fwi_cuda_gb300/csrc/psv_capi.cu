@@ -141,9 +141,7 @@ int make_survey(const psv_grid *gp, const psv_shots *sp, Survey &out)
 
 using namespace psv;
 
-// Runs job(k) for every plan on its own host thread (the plans' streams run
-// concurrently on the device) and returns the first failure.
-template <typename F> static int run_plans(psv_plan *const *plans, int n, F job)
+static int check_plans(psv_plan *const *plans, int n)
 {
     if (!plans || n <= 0) return fail(PSV_ERR_ARG, "multi: need at least one plan");
     for (int k = 0; k < n; k++) {
@@ -151,6 +149,14 @@ template <typename F> static int run_plans(psv_plan *const *plans, int n, F job)
         for (int j = 0; j < k; j++)
             if (plans[j] == plans[k]) return fail(PSV_ERR_ARG, "multi: plan listed twice");
     }
+    return PSV_OK;
+}
+
+// Runs job(k) for every plan on its own host thread (the plans' streams run
+// concurrently on the device) and returns the first failure.
+template <typename F> static int run_plans(psv_plan *const *plans, int n, F job)
+{
+    PSV_TRY(check_plans(plans, n));
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return fail(PSV_ERR_CUDA, "multi: no current device");
     std::vector<int> st(n, PSV_OK);
@@ -266,41 +272,35 @@ int psv_plan_set_observed(psv_plan *p, const double *uz, const double *ux)
 int psv_forward(psv_plan *p, double *uz, double *ux)
 {
     PLAN_CHECK(p);
+    PSV_TRY(p->impl->share(false));
     return p->impl->forward(uz, ux);
 }
 
 int psv_gradient(psv_plan *p, double *L2, double *gl, double *gm, double *gr)
 {
     PLAN_CHECK(p);
+    PSV_TRY(p->impl->share(false));
     PSV_TRY(p->impl->gradient(L2));
     if (gl || gm || gr) return p->impl->get_gradient(gl, gm, gr);
     return PSV_OK;
 }
 
-// Several plans are about to run at once.
-static int share_all(psv_plan *const *plans, int n)
-{
-    if (plans && n > 1)
-        for (int k = 0; k < n; k++)
-            if (plans[k] && plans[k]->impl) PSV_TRY(plans[k]->impl->share());
-    return PSV_OK;
-}
-
 int psv_multi_forward(psv_plan *const *plans, int n, double *const *uz, double *const *ux)
 {
-    PSV_TRY(share_all(plans, n));
     return run_plans(plans, n, [&](int k) {
+        PSV_TRY(plans[k]->impl->share(n > 1));
         return plans[k]->impl->forward(uz ? uz[k] : nullptr, ux ? ux[k] : nullptr);
     });
 }
 
 int psv_multi_gradient(psv_plan *const *plans, int n, double *L2)
 {
-    PSV_TRY(share_all(plans, n));
-    if (plans && n > 0)
-        for (int k = 0; k < n; k++)  // tune serially: concurrent work would distort the timings
-            if (plans[k] && plans[k]->impl) PSV_TRY(plans[k]->impl->prepare());
-    std::vector<double> l2(n > 0 ? n : 0, 0.0);
+    PSV_TRY(check_plans(plans, n));
+    for (int k = 0; k < n; k++) {  // tune serially: concurrent work would distort the timings
+        PSV_TRY(plans[k]->impl->share(n > 1));
+        PSV_TRY(plans[k]->impl->prepare());
+    }
+    std::vector<double> l2(n, 0.0);
     PSV_TRY(run_plans(plans, n, [&](int k) { return plans[k]->impl->gradient(&l2[k]); }));
     if (L2)
         for (int k = 0; k < n; k++) L2[k] = l2[k];
@@ -336,6 +336,7 @@ int psv_fwi_iteration(psv_plan *p, double *step, double *L2, int *ntrials, doubl
 {
     PLAN_CHECK(p);
     if (!step || !(*step > 0)) return fail(PSV_ERR_ARG, "step estimate must be > 0");
+    PSV_TRY(p->impl->share(false));
     return p->impl->fwi_iteration(step, L2, ntrials, tlog, maxt);
 }
 
@@ -425,6 +426,7 @@ int psv_plan_autotune(psv_plan *p, int nsteps, int *family, int *rpt, int *by)
 {
     PLAN_CHECK(p);
     if (nsteps <= 0) return fail(PSV_ERR_ARG, "autotune: nsteps must be positive");
+    PSV_TRY(p->impl->share(false));
     return p->impl->autotune(nsteps, family, rpt, by);
 }
 
@@ -454,6 +456,7 @@ int psv_profile_kernels(psv_plan *p, int nsteps, double *ms6)
 {
     PLAN_CHECK(p);
     if (!ms6) return fail(PSV_ERR_ARG, "null output");
+    PSV_TRY(p->impl->share(false));
     return p->impl->profile(nsteps, ms6);
 }
 
@@ -473,6 +476,7 @@ int psv_trial_misfit(psv_plan *p, double step, double *L2)
 {
     PLAN_CHECK(p);
     if (!L2) return fail(PSV_ERR_ARG, "null L2 output");
+    PSV_TRY(p->impl->share(false));
     return p->impl->trial_misfit(step, L2);
 }
 

@@ -212,6 +212,13 @@ struct DevMem {
     DevMem() = default;
     DevMem(const DevMem &) = delete;
     DevMem &operator=(const DevMem &) = delete;
+    DevMem(DevMem &&o) noexcept { *this = std::move(o); }
+    DevMem &operator=(DevMem &&o) noexcept  // swaps
+    {
+        std::swap(p, o.p);
+        std::swap(bytes, o.bytes);
+        return *this;
+    }
     ~DevMem() { release(); }
     void release()
     {
@@ -267,7 +274,8 @@ struct PlanIface {
     virtual void shape(int *fam, int *rpt, int *by) const = 0;
     virtual void storage(int *kind, int *segment_steps, int *slots, long long *advances) const = 0;
     virtual int chain_count() const = 0;
-    virtual int share() = 0;    // other plans run at the same time (psv_multi_*)
+    // Whether the passes that follow run beside other plans' (psv_multi_*).
+    virtual int share(bool on) = 0;
     virtual int prepare() = 0;  // history buffers and the pending autotune, before concurrent use
     // Joint forward modelling (psv_joint.cu): switch to the direct family with
     // rpt rows per thread and 32 x by blocks, select shot batch `batch`, zero

@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 
 #include "psv_checkpoint.hpp"
 #include "psv_plan.cuh"
@@ -47,8 +48,26 @@ enum PassKind {
     NPASS = 5
 };
 
+// The kernels of the time step and what is built for them.
+struct Shape {
+    int fam = PSV_KERNELS_DIRECT;  // kernel family; 0: not chosen yet
+    int rpt = 1;                   // rows per thread (< 0: shuffle variant)
+    dim3 blk{32, 8, 1};
+    int chains = 1;
+    bool tuned = false;
+    TileMaps tmap{}, tmap2{};    // tensor maps of fld / fld2 (TMA family)
+    LoopMaps lmap{}, lmap2{};    // ... and of its many-step launches
+    MarchMaps mmap{}, mmap2{};   // ... (MARCH family)
+    DevMem t_src_off, t_src_k, t_rec_off, t_rec_r;  // per-tile source / receiver index
+    int ntiles = 0;
+    DevMem lkeep, lkept;         // per tile: keeps its sums' roundings; those tiles
+    int nkept = 0;
+    cudaGraphExec_t gx[NPASS] = {};
+    long long gx_nodes[NPASS] = {};  // kernels in each captured pass
+};
+
 template <typename T>
-class Plan final : public PlanIface {
+class Plan final : public PlanIface, Shape {
 public:
     Survey sv;
     psv_options opt;
@@ -64,17 +83,9 @@ public:
     DevMem fld, memz, memx, hist, gshot, coef, prof, fsb;
     DevMem model, stf, traces, red, taperb, ctl, scales;
     DevMem f_off, f_pos, f_col, f_snap, a_off, a_pos, a_col, a_snap, rec_pos;
-    DevMem t_src_off, t_src_k, t_rec_off, t_rec_r;  // per-tile source / receiver index
-    int rpt = 1;                                     // rows per thread (< 0: shuffle variant)
-    int fam = PSV_KERNELS_DIRECT;                    // kernel family of the time step
-    TileMaps tmap{}, tmap2{};                        // tensor maps of fld / fld2 (TMA family)
-    LoopMaps lmap{}, lmap2{};                        // ... and of its many-step launches
     ResidentTile rt{};                               // tiles of the resident kernel (tz = 0: does not serve)
     DevMem lsync;                                    // item counter and progress words, or the tiles' inboxes
-    DevMem lkeep, lkept;                             // per tile: keeps its sums' roundings; those tiles
-    int nkept = 0;
     long long ck_kept = 0;  // elements of a checkpointed state that hold them
-    MarchMaps mmap{}, mmap2{};                       // tensor maps of fld / fld2 (MARCH family)
     int *h_err = nullptr;                            // pinned copy of the device error word
     std::vector<int> h_f_off;                        // host copy of the per-shot source lists
     // Checkpointed storage: nck state slots at starts of K-step segments
@@ -94,7 +105,6 @@ public:
     DevMem ck, fld2, memz2, memx2;
     StepParams<T> sp{}, sp2{};
     SrcRecParams<T> qf{}, qa{}, qk{}, qr{};
-    cudaGraphExec_t gx[NPASS] = {};
     double C[3] = {0, 0, 0};
     double inj = 1.0;     // dt/(dz dx) * max(1/rho): injection gain of a displacement source
     double gscale = 1.0;  // power of two on the imaging factors g1, g2
@@ -102,16 +112,13 @@ public:
     int last_s0 = -1, last_n = 0, last_batch_s0 = 0;
     double t_ms[3] = {0, 0, 0};
     bool have_model = false, have_obs = false, store_flag = false;
-    bool tuned = false;
-    bool beside = false;  // runs at the same time as other plans (psv_multi_*)
+    bool beside = false;  // the shape in use is the one beside other plans (psv_multi_*)
+    Shape other;          // ... the one not in use: beside others, or the plan's own
     long long nlaunch = 0;          // kernels launched (graph nodes counted per replay)
-    long long gx_nodes[NPASS] = {}; // kernels in each captured pass
-    dim3 blk{32, 8, 1};
     // Chained schedule (direct family): the batch split into `chains` groups
     // of slots whose time loops run on their own (captured) streams, so one
     // group's launches fill the kernel boundaries of the others.
     static constexpr int MAXCH = 4;
-    int chains = 1;
     cudaStream_t stc[MAXCH] = {};
     cudaEvent_t evf = nullptr, evj[MAXCH] = {};
     DevMem ctl2;            // [MAXCH][2]: global shot of the group's slot 0, shots
@@ -125,8 +132,9 @@ public:
             if (stc[k]) cudaStreamDestroy(stc[k]);
         }
         if (h_ctl2) cudaFreeHost(h_ctl2);
-        for (auto &g : gx)
-            if (g) cudaGraphExecDestroy(g);
+        drop_graphs();
+        std::swap(static_cast<Shape &>(*this), other);
+        drop_graphs();
         for (auto &e : ev)
             if (e) cudaEventDestroy(e);
         if (h_ctl) cudaFreeHost(h_ctl);
@@ -156,7 +164,6 @@ public:
     double *fscale() const { return scales.as<double>(); }
     double *funscale() const { return fscale() + sv.s.nshot; }
     double *ascale() const { return fscale() + 2 * sv.s.nshot; }
-    int ntiles = 0;
     std::vector<int> src_list_col;  // source index of each entry of the per-shot lists
     unsigned long long *rmax() const { return (unsigned long long *)(fscale() + 3 * sv.s.nshot); }
 
@@ -332,6 +339,8 @@ public:
         PSV_CU(cudaMallocHost(&h_ctl2, sizeof(int) * 2 * MAXCH * nbatch));
         chains = opt.chains == 2 || opt.chains == 4 ? opt.chains : 1;
         PSV_TRY(set_chains(chains));
+        other.fam = 0;
+        other.chains = chains;
         *h_err = 0;
         for (int b = 0; b < nbatch; b++) {
             h_ctl[2 * b] = b * B;
@@ -520,18 +529,29 @@ public:
         *r = 1;
         return PSV_KERNELS_DIRECT;
     }
-    // Runs beside other plans from now on.  The resident kernel waits until
-    // the GPU has room for all its CTAs and shares it with nobody else that
-    // fills it: four surveys at once took 21.3 ms with it, 16.6 with kernels
-    // that mix.
-    int share() override
+    // Whether the passes that follow run beside other plans'.  The resident
+    // kernel waits until the GPU has room for all its CTAs and shares it with
+    // nobody else that fills it: four surveys at once took 21.3 ms with it, 16.6
+    // with kernels that mix.  So a plan that runs it, or may be tuned to, has a
+    // second shape for those passes, chosen and built once; going from one to the
+    // other moves pointers, and each keeps its graphs.
+    int share(bool on) override
     {
-        if (beside || !any_kernels()) return PSV_OK;
-        beside = true;
-        if (!resident()) return PSV_OK;
-        tuned = false;
+        if (on == beside) return PSV_OK;
+        if (on && !(any_kernels() && rt.tz && (resident() || (opt.autotune && !tuned)))) return PSV_OK;
+        beside = on;
+        std::swap(static_cast<Shape &>(*this), other);
+        point_index();
+        group_chains();
+        return PSV_OK;
+    }
+    // The shape a pass starts with if nothing has chosen one.
+    int settle()
+    {
+        if (fam) return PSV_OK;
+        if (!any_kernels()) return set_shape(opt.kernel_family ? opt.kernel_family : PSV_KERNELS_DIRECT, rpt, (int)blk.y);
         int r, f = start_shape(&r);
-        return set_shape(f, r, opt.block_y > 0 ? opt.block_y : 8);
+        return set_shape(f, r, opt.block_y > 0 ? opt.block_y : 4);
     }
 
     // Tensor maps of the field blocks for the TMA family (rebuilt when the
@@ -957,9 +977,13 @@ public:
             sp2.memx = memx2.as<T>();
         }
         sp2.hist = hist.as<T>() + snx_off;
-        PSV_TRY(encode_maps());
-        drop_graphs();
-        return PSV_OK;
+        int rc[2];
+        for (int k = 0; k < 2; k++) {  // both shapes
+            rc[k] = encode_maps();
+            drop_graphs();
+            std::swap(static_cast<Shape &>(*this), other);
+        }
+        return rc[0] != PSV_OK ? rc[0] : rc[1];
     }
 
     // Copy the batch's forward state between checkpoint slot j and the main
@@ -1131,6 +1155,7 @@ public:
 
     int run_pass(int kind)
     {
+        PSV_TRY(settle());
         const bool graphable = kind == PASS_FWD_STORE || kind == PASS_FWD_PLAIN || kind == PASS_ADJ_RES;
         if (!opt.use_graphs || !graphable) return enqueue(kind);
         if (!gx[kind]) {
@@ -1164,6 +1189,12 @@ public:
     {
         chains = std::max(1, std::min(k, (int)MAXCH));
         while (chains > B) chains /= 2;  // 4 -> 2 -> 1: at least one shot a group
+        group_chains();
+        drop_graphs();
+        return PSV_OK;
+    }
+    void group_chains()
+    {
         const int h = (B + chains - 1) / chains;
         for (int b = 0; b < nbatch; b++) {
             const int n = std::min(B, sv.s.nshot - b * B);
@@ -1172,8 +1203,6 @@ public:
                 h_ctl2[(b * MAXCH + c) * 2 + 1] = c < chains ? std::max(0, std::min(h, n - c * h)) : 0;
             }
         }
-        drop_graphs();
-        return PSV_OK;
     }
 
     int set_batch(int b)
@@ -1674,6 +1703,16 @@ public:
         return PSV_OK;
     }
 
+    // The source / receiver index of the shape in use.
+    void point_index()
+    {
+        qf.t_src_off = qr.t_src_off = qk.t_src_off = qa.t_src_off = t_src_off.as<int>();
+        qf.t_src_k = qr.t_src_k = qk.t_src_k = qa.t_src_k = t_src_k.as<int>();
+        qf.t_rec_off = qr.t_rec_off = qk.t_rec_off = qa.t_rec_off = t_rec_off.as<int>();
+        qf.t_rec_r = qr.t_rec_r = qk.t_rec_r = qa.t_rec_r = t_rec_r.as<int>();
+        qf.ntiles = qr.ntiles = qk.ntiles = qa.ntiles = ntiles;
+    }
+
     // Switch the stencil kernels' tile shape (rebuilds the per-tile source
     // index, drops captured graphs).
     int set_shape(int f, int r, int by)
@@ -1694,15 +1733,12 @@ public:
         fam = f;
         rpt = r;
         blk = dim3(32, by, 1);
-        PSV_TRY(build_tile_index());
-        qf.t_src_off = qr.t_src_off = qk.t_src_off = qa.t_src_off = t_src_off.as<int>();
-        qf.t_src_k = qr.t_src_k = qk.t_src_k = qa.t_src_k = t_src_k.as<int>();
-        qf.t_rec_off = qr.t_rec_off = qk.t_rec_off = qa.t_rec_off = t_rec_off.as<int>();
-        qf.t_rec_r = qr.t_rec_r = qk.t_rec_r = qa.t_rec_r = t_rec_r.as<int>();
-        qf.ntiles = qr.ntiles = qk.ntiles = qa.ntiles = ntiles;
-        PSV_TRY(encode_maps());
+        int rc = build_tile_index();
+        point_index();
+        if (rc == PSV_OK) rc = encode_maps();
         drop_graphs();
-        return PSV_OK;
+        if (rc != PSV_OK) fam = 0;  // half built: the next pass chooses again
+        return rc;
     }
 
     int autotune(int nsteps, int *out_fam, int *out_rpt, int *out_by) override
@@ -1813,11 +1849,13 @@ public:
         if (advances) *advances = ckpt ? sched.advances : 0;
     }
 
+    // (one not chosen yet is not reported)
     void shape(int *f, int *r, int *by) const override
     {
-        if (f) *f = fam;
-        if (r) *r = rpt;
-        if (by) *by = fam == PSV_KERNELS_TMA ? 4 : fam == PSV_KERNELS_FUSED ? 0 : (int)blk.y;
+        const Shape &s = fam ? static_cast<const Shape &>(*this) : other;
+        if (f) *f = s.fam;
+        if (r) *r = s.rpt;
+        if (by) *by = s.fam == PSV_KERNELS_TMA ? 4 : s.fam == PSV_KERNELS_FUSED ? 0 : (int)s.blk.y;
     }
 
     int prepare() override
@@ -1836,6 +1874,7 @@ public:
             return fail(PSV_ERR_ARG, "joint launch: every plan of one precision");
         if (!have_model) return fail(PSV_ERR_ARG, "joint launch: a plan has no model");
         if (batch < 0 || batch >= nbatch) return fail(PSV_ERR_ARG, "joint launch: no such shot batch");
+        PSV_TRY(share(false));
         PSV_TRY(set_shape(PSV_KERNELS_DIRECT, r, by));
         if (fam != PSV_KERNELS_DIRECT || rpt != r || (int)blk.y != by)
             return fail(PSV_ERR_ARG, "joint launch: unsupported tile shape");
@@ -1944,6 +1983,7 @@ public:
             if (opt.adjoint == PSV_ADJOINT_EXACT)
                 return fail(PSV_ERR_UNSUPPORTED, "joint gradient: the reference-mode adjoint only");
             if (batch < 0 || batch >= nbatch) return fail(PSV_ERR_ARG, "joint launch: no such shot batch");
+            PSV_TRY(share(false));
             if (batch == 0) {
                 PSV_TRY(ensure_hist());
                 PSV_TRY(coefficients(true, false));
@@ -2076,6 +2116,7 @@ public:
     {
         if (!have_model || !have_obs) return fail(PSV_ERR_ARG, "profile: model and observed traces required");
         if (nsteps <= 0 || nsteps > sv.g.nt) return fail(PSV_ERR_ARG, "profile: nsteps must be in [1, nt]");
+        PSV_TRY(settle());
         PSV_TRY(ensure_hist());
         PSV_TRY(coefficients(true, false));
         PSV_TRY(set_batch(0));

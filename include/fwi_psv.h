@@ -239,6 +239,8 @@ int psv_gradient(psv_plan *plan, double *L2, double *grad_lam, double *grad_mu,
  * on its plan's own stream and host thread, so the GPU overlaps the surveys'
  * time loops; one call, not one kernel launch.  Plans still due an autotune
  * are tuned one after another first, so their timings are not disturbed.
+ * A plan whose own kernels need the whole GPU at once (small batches) has
+ * others for these calls; what it runs alone does not change.
  * The same plan may not appear twice.  forward: uz[k], ux[k] as in
  * psv_forward for plan k (entries may be NULL); gradient: L2[k] per plan
  * (may be NULL), the global gradients stay on each plan (psv_get_gradient).
@@ -428,8 +430,9 @@ int psv_last_timing(const psv_plan *plan, double *ms3);
  * NULL). */
 int psv_plan_autotune(psv_plan *plan, int nsteps, int *kernel_family, int *rows_per_thread,
                       int *block_y);
-/* The time-step kernels the plan launches now: family (PSV_KERNELS_*), rows
- * per thread (FUSED: tile rows, MARCH: rows a CTA marches) and block height
+/* The time-step kernels the plan launches now (after psv_multi_*: the ones it
+ * had there, until its next call alone): family (PSV_KERNELS_*), rows per
+ * thread (FUSED: tile rows, MARCH: rows a CTA marches) and block height
  * (TMA: 4, FUSED: 0, MARCH: warps per CTA); any pointer may be NULL. */
 int psv_plan_shape(const psv_plan *plan, int *kernel_family, int *rows_per_thread, int *block_y);
 /* Shot groups (streams) the plan's time loops run in: 1, 2 or 4. */
