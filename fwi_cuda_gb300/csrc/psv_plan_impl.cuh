@@ -227,26 +227,24 @@ public:
             return fail(PSV_ERR_UNSUPPORTED, "grid too large: one shot's field planes exceed "
                                              "2^31 - 1 elements (nz x padded nx x " +
                                                  std::to_string(nfield()) + " planes)");
-        if (sizeof(T) == 4 && g.pml_x) {
-            // x strips that start and end on multiples of four columns: the
-            // added columns' profiles are the identity, and 128-bit accesses
-            // then fall inside a strip or outside it
-            sv.px0 = (sv.px0 + 3) & ~3;
-            if (sv.px1 < nx) sv.px1 &= ~3;
-            if (sv.px0 >= sv.px1) sv.px0 = sv.px1 = nx;  // all strip
-        }
-        nzs = g.pml_z ? sv.pz0 + (nz - sv.pz1) : 0;
-        nxs = g.pml_x ? sv.px0 + (nx - sv.px1) : 0;
-        mx_pitch = nxs ? round_up(nxs, al) : 0;
-        mz_shot = (long long)(sizeof(T) == 4 ? NMZ_PP : NMZ) * nzs * pitch;
-        mx_shot = (long long)(sizeof(T) == 4 ? NMX_PP : NMX) * nz * mx_pitch;
-        // Stored rows start so that a window column has its grid column's
-        // alignment (128-bit stores and loads of whole quads).
-        snx_off = sizeof(T) == 4 && g.snap_dx == 1 ? g.snap_x1 & 3 : 0;
-        snx_pitch = round_up(sv.snx + snx_off, al);
-        const long long snap_plane = (long long)sv.snz * snx_pitch;
-        hist_shot = (long long)sv.snt * NHIST * snap_plane;
-        gshot_shot = 3 * snap_plane;
+        // What fits the budget is decided on rows as they are without the alignment
+        // that the FP32 kernels' 128-bit accesses want; they are laid out again with
+        // it afterwards, at most eight elements longer.
+        long long snap_plane = 0;
+        auto layout = [&](int strip_row, int snap_row) {
+            nzs = g.pml_z ? sv.pz0 + (nz - sv.pz1) : 0;
+            nxs = g.pml_x ? sv.px0 + (nx - sv.px1) : 0;
+            mx_pitch = strip_row;
+            mz_shot = (long long)(sizeof(T) == 4 ? NMZ_PP : NMZ) * nzs * pitch;
+            mx_shot = (long long)(sizeof(T) == 4 ? NMX_PP : NMX) * nz * mx_pitch;
+            snx_pitch = snap_row;
+            snap_plane = (long long)sv.snz * snx_pitch;
+            hist_shot = (long long)sv.snt * NHIST * snap_plane;
+            gshot_shot = 3 * snap_plane;
+            ck_state = 5 * plane + mz_shot + mx_shot;
+        };
+        const int strips = g.pml_x ? sv.px0 + (nx - sv.px1) : 0;
+        layout(strips ? round_up(strips, al) : 0, round_up(sv.snx, al));
         ntr = (long long)g.nt * nrec;
 
         const double budget = (opt.hbm_budget_gb > 0 ? opt.hbm_budget_gb : 180.0) * 1e9;
@@ -254,7 +252,6 @@ public:
         const double per_hist = (double)hist_shot * sizeof(T);
         const double shared = 7.0 * plane * sizeof(T) + 12.0 * nz * nx * 8 + 6.0 * nshot * ntr * 8;
         // checkpointed alternative: K minimising nt/K states + K/snap_dt snapshots
-        ck_state = 5 * plane + mz_shot + mx_shot;
         const double snap5 = (double)NHIST * snap_plane, sdt = g.snap_dt;
         const bool binomial = opt.storage == PSV_STORE_BINOMIAL;
         auto segments = [&](int k) {
@@ -262,50 +259,64 @@ public:
             nseg = (g.nt + K - 1) / K;
             nslots = (K + g.snap_dt - 1) / g.snap_dt + 1;
         };
-        segments(opt.checkpoint_interval > 0 ? opt.checkpoint_interval
-                 : binomial ? g.snap_dt
-                            : (int)std::max(1.0, std::round(std::sqrt(g.nt * (double)ck_state * sdt / snap5))));
-        auto per_ck = [&](int slots) {
-            return ((double)slots * ck_state + (double)ck_state + (double)nslots * snap5) * sizeof(T);
-        };
-        auto fit = [&](double extra) {
-            int b = opt.max_batch > 0 ? std::min(opt.max_batch, nshot) : nshot;
-            while (b > 1 && shared + b * (per_shot + extra) > budget) b--;
-            return shared + b * (per_shot + extra) <= budget ? b : 0;
-        };
-        if (sizeof(T) == 4)  // a state also holds the kept roundings of the looped tiles
-            ck_kept = 5 * 64 * (long long)std::max(8 * kept_tiles(8).size(), 16 * kept_tiles(16).size());
-        ck_state += ck_kept;
-        const int b_full = fit(per_hist);
-        int b_ck = binomial ? 0 : fit(per_ck(nseg));
-        nck = nseg;
-        if (opt.storage == PSV_STORE_FULL) {
-            if (!b_full) return fail(PSV_ERR_OOM, "full snapshot history of one shot exceeds the HBM budget");
-            B = b_full;
-        } else if (opt.storage == PSV_STORE_CHECKPOINT) {
-            if (!b_ck) return fail(PSV_ERR_OOM, "checkpoints of one shot exceed the HBM budget");
-            ckpt = true;
-            B = b_ck;
-        } else if (!binomial && (b_full || b_ck)) {
-            ckpt = b_ck > b_full;
-            B = ckpt ? b_ck : b_full;
-        } else {
-            // binomial: the slots asked for, else the fewest giving at most two
-            // forward repetitions (C(S + 2, 2) >= nseg), at the largest batch
-            // that holds them; with less room, one shot and every slot that fits
-            if (!binomial && opt.checkpoint_interval <= 0) segments(g.snap_dt);
-            int S = opt.checkpoint_slots > 0 ? opt.checkpoint_slots : 1;
-            if (opt.checkpoint_slots <= 0)
-                while (S < nseg && ck_reps(nseg, S) > 2) S++;
-            S = std::min(S, nseg);
-            B = fit(per_ck(S));
-            if (!B && opt.checkpoint_slots <= 0) {
-                while (S > 2 && !fit(per_ck(S))) S--;
+        // Storage kind, batch, segments and slots with `kept` elements more a state.
+        auto decide = [&](long long kept) -> int {
+            segments(opt.checkpoint_interval > 0 ? opt.checkpoint_interval
+                     : binomial ? g.snap_dt
+                                : (int)std::max(1.0, std::round(std::sqrt(g.nt * (double)ck_state * sdt / snap5))));
+            const double state = (double)(ck_state + kept);
+            auto per_ck = [&](int slots) {
+                return ((double)slots * state + state + (double)nslots * snap5) * sizeof(T);
+            };
+            auto fit = [&](double extra) {
+                int b = opt.max_batch > 0 ? std::min(opt.max_batch, nshot) : nshot;
+                while (b > 1 && shared + b * (per_shot + extra) > budget) b--;
+                return shared + b * (per_shot + extra) <= budget ? b : 0;
+            };
+            const int b_full = fit(per_hist);
+            const int b_ck = binomial ? 0 : fit(per_ck(nseg));
+            nck = nseg;
+            ckpt = false;
+            if (opt.storage == PSV_STORE_FULL) {
+                if (!b_full) return fail(PSV_ERR_OOM, "full snapshot history of one shot exceeds the HBM budget");
+                B = b_full;
+            } else if (opt.storage == PSV_STORE_CHECKPOINT) {
+                if (!b_ck) return fail(PSV_ERR_OOM, "checkpoints of one shot exceed the HBM budget");
+                ckpt = true;
+                B = b_ck;
+            } else if (!binomial && (b_full || b_ck)) {
+                ckpt = b_ck > b_full;
+                B = ckpt ? b_ck : b_full;
+            } else {
+                // binomial: the slots asked for, else the fewest giving at most two
+                // forward repetitions (C(S + 2, 2) >= nseg), at the largest batch
+                // that holds them; with less room, one shot and every slot that fits
+                if (!binomial && opt.checkpoint_interval <= 0) segments(g.snap_dt);
+                int S = opt.checkpoint_slots > 0 ? opt.checkpoint_slots : 1;
+                if (opt.checkpoint_slots <= 0)
+                    while (S < nseg && ck_reps(nseg, S) > 2) S++;
+                S = std::min(S, nseg);
                 B = fit(per_ck(S));
+                if (!B && opt.checkpoint_slots <= 0) {
+                    while (S > 2 && !fit(per_ck(S))) S--;
+                    B = fit(per_ck(S));
+                }
+                if (!B) return fail(PSV_ERR_OOM, "binomial checkpoints of one shot exceed the HBM budget");
+                ckpt = true;
+                nck = S;
             }
-            if (!B) return fail(PSV_ERR_OOM, "binomial checkpoints of one shot exceed the HBM budget");
-            ckpt = true;
-            nck = S;
+            return PSV_OK;
+        };
+        PSV_TRY(decide(0));
+        // A state also holds the roundings that tiles keep (keep_sum), where the
+        // kernels that keep them may run and the batch is not the smaller for it.
+        if (sizeof(T) == 4 && (any_kernels() || opt.kernel_family == PSV_KERNELS_TMA) && !sv.sb && !sv.sl && !sv.sr) {
+            const int most = B;
+            ck_kept = 5 * 64 * (long long)std::max(8 * kept_tiles(8).size(), 16 * kept_tiles(16).size());
+            if (decide(ck_kept) != PSV_OK || B < most) {
+                ck_kept = 0;
+                PSV_TRY(decide(0));
+            }
         }
         if (ckpt) {
             store_kind = nck < nseg ? PSV_STORE_BINOMIAL : PSV_STORE_CHECKPOINT;
@@ -316,6 +327,22 @@ public:
             sched = ck_schedule(nseg, nck);
             fwd_slot.assign((size_t)nseg, -1);
             for (const CkAction &x : sched.fwd) fwd_slot[(size_t)x.seg] = x.slot;
+        }
+        if (sizeof(T) == 4) {
+            // x strips that start and end on multiples of four columns: the
+            // added columns' profiles are the identity, and 128-bit accesses
+            // then fall inside a strip or outside it
+            if (g.pml_x) {
+                sv.px0 = (sv.px0 + 3) & ~3;
+                if (sv.px1 < nx) sv.px1 &= ~3;
+                if (sv.px0 >= sv.px1) sv.px0 = sv.px1 = nx;  // all strip
+            }
+            // Stored rows start so that a window column has its grid column's
+            // alignment (128-bit stores and loads of whole quads).
+            snx_off = g.snap_dx == 1 ? g.snap_x1 & 3 : 0;
+            auto grown = [&](int row, int n) { return n <= row ? row : round_up(n, 8); };
+            layout(grown(mx_pitch, g.pml_x ? sv.px0 + (nx - sv.px1) : 0), grown(snx_pitch, sv.snx + snx_off));
+            ck_state += ck_kept;
         }
         if (ckpt) hist_shot = (long long)nslots * NHIST * snap_plane;
         nbatch = (nshot + B - 1) / B;
@@ -447,7 +474,7 @@ public:
     int build_kept()
     {
         nkept = 0;
-        if (!looped()) return PSV_OK;
+        if (!looped() || (ckpt && !ck_kept)) return PSV_OK;
         const int tz = kept_rows();
         const std::vector<int> t = kept_tiles(tz);
         std::vector<int> on((size_t)((sv.g.nx + 63) / 64) * ((sv.g.nz + tz - 1) / tz), 0);
