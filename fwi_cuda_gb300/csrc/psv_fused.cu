@@ -318,9 +318,9 @@ cudaError_t launch_fused_m(const StepParams<float> &p, const SrcRecParams<float>
                            int slot, int par, int nbatch, cudaStream_t st)
 {
     using G = FusedGeo<NS, TZ>;
-    static cudaError_t attr = cudaFuncSetAttribute(
-        k_step_fused<NS, MODE, TZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-    if (attr != cudaSuccess) return attr;
+    static PerDevice<cudaError_t> opted;
+    const cudaError_t e = opt_in(opted, k_step_fused<NS, MODE, TZ>, G::SMEM);
+    if (e != cudaSuccess) return e;
     const dim3 grid((p.nx + FTX - 1) / FTX, (p.nz + TZ - 1) / TZ, nbatch);
     k_step_fused<NS, MODE, TZ><<<grid, FNT, G::SMEM, st>>>(p, q, it, slot, par);
     return cudaGetLastError();

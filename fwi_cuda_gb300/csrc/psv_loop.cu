@@ -790,7 +790,9 @@ cudaError_t loop_m(const StepParams<float> &p, const SrcRecParams<float> &q, con
         cudaError_t e;
         int ctas;
     };
-    static const Fit fit = [&] {  // per instantiation: CTAs the GPU holds at once
+    static PerDevice<Fit> fits;  // per instantiation: CTAs the GPU holds at once
+    Fit fit{cudaSuccess, 0};
+    cudaError_t e = on_device(fits, [&] {
         Fit r{cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), 0};
         int per = 0, dev = 0, nsm = 0;
         if (r.e == cudaSuccess) r.e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, (loop_threads<NS, TZ>()), smem);
@@ -799,10 +801,11 @@ cudaError_t loop_m(const StepParams<float> &p, const SrcRecParams<float> &q, con
         if (r.e == cudaSuccess && per < 1) r.e = cudaErrorInvalidConfiguration;
         r.ctas = per * nsm;
         return r;
-    }();
-    if (fit.e != cudaSuccess) return fit.e;
+    }, &fit);
+    if (e == cudaSuccess) e = fit.e;
+    if (e != cudaSuccess) return e;
     const int tiles = ((p.nx + TW - 1) / TW) * ((p.nz + TZ - 1) / TZ) * nbatch;
-    cudaError_t e = cudaMemsetAsync(run.sync, 0, (size_t)(LOOP_SYNC_HEAD + tiles * FLAG_STRIDE) * sizeof(int), st);
+    e = cudaMemsetAsync(run.sync, 0, (size_t)(LOOP_SYNC_HEAD + tiles * FLAG_STRIDE) * sizeof(int), st);
     if (e != cudaSuccess) return e;
     kernel<<<std::min(fit.ctas, tiles), loop_threads<NS, TZ>(), smem, st>>>(p, q, m, run);
     return cudaGetLastError();

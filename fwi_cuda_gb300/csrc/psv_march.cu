@@ -313,9 +313,9 @@ cudaError_t launch_march_m(const StepParams<float> &p, const SrcRecParams<float>
                            cudaStream_t st)
 {
     using G = MGeo<NS, R>;
-    static cudaError_t attr = cudaFuncSetAttribute(
-        k_step_march<NS, MODE, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-    if (attr != cudaSuccess) return attr;
+    static PerDevice<cudaError_t> opted;
+    const cudaError_t e = opt_in(opted, k_step_march<NS, MODE, R>, G::SMEM);
+    if (e != cudaSuccess) return e;
     const dim3 grid(nbatch, (p.nx + G::W - 1) / G::W, (p.nz + L - 1) / L);
     k_step_march<NS, MODE, R><<<grid, MTHREADS, G::SMEM, st>>>(p, q, mm, it, slot, par, L);
     return cudaGetLastError();

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "fwi_psv.h"
+#include "psv_device.hpp"
 #include "psv_fwi.cuh"
 #include "psv_internal.h"
 #include "psv_kernels.cuh"
@@ -183,6 +184,23 @@ cudaError_t launch_velocity_tma(const StepParams<float> &p, const SrcRecParams<f
         if (e_ != cudaSuccess)                                                              \
             return ::psv::fail(PSV_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
+
+// The value of `v` on the current device.
+template <typename V, typename F> cudaError_t on_device(PerDevice<V> &v, F make, V *out)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) *out = v.get(dev, make);
+    return e;
+}
+// Opts the kernel into `smem` bytes of dynamic shared memory on the current device.
+template <typename K> cudaError_t opt_in(PerDevice<cudaError_t> &v, K kernel, int smem)
+{
+    cudaError_t r = cudaSuccess;
+    const cudaError_t e = on_device(
+        v, [&] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); }, &r);
+    return e != cudaSuccess ? e : r;
+}
 
 #define PSV_TRY(call)                  \
     do {                               \

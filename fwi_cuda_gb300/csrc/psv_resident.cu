@@ -591,11 +591,11 @@ cudaError_t resident_m(const StepParams<float> &p, const SrcRecParams<float> &q,
 {
     constexpr int RW = 32 * QPT;
     auto kernel = k_resident<NS, QPT, MODE>;
-    static const cudaError_t opt_in = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                           resident_smem(NS, RW, MAX_THREADS / 8));
-    if (opt_in != cudaSuccess) return opt_in;
+    static PerDevice<cudaError_t> opted;
+    cudaError_t e = opt_in(opted, kernel, resident_smem(NS, RW, MAX_THREADS / 8));
+    if (e != cudaSuccess) return e;
     const int ctas = g.ntx * g.ntz * nbatch;
-    cudaError_t e = cudaMemsetAsync(g.inbox, 0, (size_t)ctas * 2 * rim_cells(NS, RW, g.tz) * sizeof(ulonglong2), st);
+    e = cudaMemsetAsync(g.inbox, 0, (size_t)ctas * 2 * rim_cells(NS, RW, g.tz) * sizeof(ulonglong2), st);
     if (e != cudaSuccess) return e;
     StepParams<float> a = p;
     SrcRecParams<float> s = q;

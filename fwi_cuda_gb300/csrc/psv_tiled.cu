@@ -544,12 +544,15 @@ template <typename K> Occupancy occupancy(K kernel, int smem)
 }
 
 // Persistent grid: as many CTAs as fit on the GPU at once, at most one per tile.
-cudaError_t pipe_grid(const Occupancy &o, int ntile, int *grid)
+template <typename K> cudaError_t pipe_grid(PerDevice<Occupancy> &occ, K kernel, int smem, int ntile, int *grid)
 {
-    if (o.e != cudaSuccess) return o.e;
+    Occupancy o{cudaSuccess, 0};
+    cudaError_t e = on_device(occ, [&] { return occupancy(kernel, smem); }, &o);
+    if (e == cudaSuccess) e = o.e;
+    if (e != cudaSuccess) return e;
     if (o.per_sm < 1) return cudaErrorInvalidConfiguration;
     int dev = 0, nsm = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     *grid = std::max(1, std::min(ntile, nsm * o.per_sm));
@@ -561,9 +564,9 @@ cudaError_t stress_rn(const StepParams<float> &p, const TileMaps &m, int nbatch,
 {
     constexpr int smem = pipe_smem_bytes(2, 6, NS, R);
     const int ntile = ((p.nx + TW - 1) / TW) * ((p.nz + 4 * R - 1) / (4 * R)) * nbatch;
-    static const Occupancy occ = occupancy(k_stress_tma<NS, R>, smem);  // per instantiation
+    static PerDevice<Occupancy> occ;  // per instantiation
     int grid = 0;
-    const cudaError_t e = pipe_grid(occ, ntile, &grid);
+    const cudaError_t e = pipe_grid(occ, k_stress_tma<NS, R>, smem, ntile, &grid);
     if (e != cudaSuccess) return e;
     k_stress_tma<NS, R><<<grid, NTHREADS, smem, st>>>(p, m);
     return cudaGetLastError();
@@ -587,9 +590,9 @@ cudaError_t velocity_rmn(const StepParams<float> &p, const SrcRecParams<float> &
 {
     constexpr int smem = pipe_smem_bytes(3, vel_own_planes<MODE>(true), NS, R);
     const int ntile = ((p.nx + TW - 1) / TW) * ((p.nz + 4 * R - 1) / (4 * R)) * nbatch;
-    static const Occupancy occ = occupancy(k_velocity_tma<NS, MODE, R>, smem);  // per instantiation
+    static PerDevice<Occupancy> occ;  // per instantiation
     int grid = 0;
-    const cudaError_t e = pipe_grid(occ, ntile, &grid);
+    const cudaError_t e = pipe_grid(occ, k_velocity_tma<NS, MODE, R>, smem, ntile, &grid);
     if (e != cudaSuccess) return e;
     k_velocity_tma<NS, MODE, R><<<grid, NTHREADS, smem, st>>>(p, q, it, slot, m);
     return cudaGetLastError();

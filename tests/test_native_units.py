@@ -8,7 +8,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-@pytest.mark.parametrize("unit", ["surface_rows"])
+@pytest.mark.parametrize("unit", ["surface_rows", "per_device"])
 def test_unit(tmp_path, unit):
     cxx = shutil.which("g++") or shutil.which("c++")
     if not cxx:
