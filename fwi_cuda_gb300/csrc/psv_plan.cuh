@@ -81,6 +81,7 @@ struct ResidentTile {
     int rw, tz;
 };
 ResidentTile resident_tile(int nz, int nx, int nbatch, int ns, int st, int sb, int sl, int sr, int nz1, int nsm);
+bool resident_held(int nz, int nx, int nbatch, int ns, const ResidentTile &t, int nsm);
 size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, const ResidentTile &t);
 cudaError_t launch_resident(const StepParams<float> &p, const SrcRecParams<float> &q, const LoopRun &run, int ns,
                             int mode, const ResidentTile &t, int nbatch, cudaStream_t st);

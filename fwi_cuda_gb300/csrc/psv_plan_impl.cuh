@@ -352,6 +352,7 @@ public:
             PSV_CU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
             PSV_CU(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
             if (coop) rt = resident_tile(nz, nx, B, sv.ns, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1, nsm);
+            if (rt.tz && !resident_held(nz, nx, B, sv.ns, rt, nsm)) rt = {0, 0};
         }
         if (any_kernels()) fam = start_shape(&rpt);
 

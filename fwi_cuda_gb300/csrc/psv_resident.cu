@@ -585,6 +585,31 @@ __global__ void __launch_bounds__(MAX_THREADS, 1)
     }
 }
 
+// Lowers *held to the CTAs of tz rows that the current device holds at once.
+template <int NS, int QPT, int MODE> cudaError_t held_m(int tz, int nsm, int *held)
+{
+    constexpr int RW = 32 * QPT;
+    auto kernel = k_resident<NS, QPT, MODE>;
+    static PerDevice<cudaError_t> opted;
+    int per = 0;
+    cudaError_t e = opt_in(opted, kernel, resident_smem(NS, RW, MAX_THREADS / 8));
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, resident_threads(NS, RW, tz),
+                                                          resident_smem(NS, RW, tz));
+    *held = e == cudaSuccess ? std::min(*held, per * nsm) : 0;
+    return e;
+}
+template <int NS, int QPT> int held_q(int tz, int nsm)
+{
+    int held = 1 << 30;
+    const cudaError_t e[] = {held_m<NS, QPT, MODE_FWD>(tz, nsm, &held), held_m<NS, QPT, MODE_FWD_NOWE>(tz, nsm, &held),
+                             held_m<NS, QPT, MODE_FWD_U>(tz, nsm, &held), held_m<NS, QPT, MODE_ADJ>(tz, nsm, &held)};
+    for (cudaError_t x : e)
+        if (x != cudaSuccess) held = 0;
+    if (!held) (void)cudaGetLastError();
+    return held;
+}
+
 template <int NS, int QPT, int MODE>
 cudaError_t resident_m(const StepParams<float> &p, const SrcRecParams<float> &q, const ResidentRun &g, int nbatch,
                        cudaStream_t st)
@@ -648,6 +673,21 @@ ResidentTile resident_tile(int nz, int nx, int nbatch, int ns, int st, int sb, i
             }
     }
     return {0, 0};
+}
+
+// Whether the current device holds all CTAs of a batch at once, by its own
+// account: a launch that it cannot hold is refused.
+bool resident_held(int nz, int nx, int nbatch, int ns, const ResidentTile &t, int nsm)
+{
+    const long long ctas = (long long)((nx + t.rw - 1) / t.rw) * ((nz + t.tz - 1) / t.tz) * nbatch;
+    int held = 0;
+    switch (ns) {
+    case 1: held = t.rw == 32 ? held_q<1, 1>(t.tz, nsm) : held_q<1, 2>(t.tz, nsm); break;
+    case 2: held = t.rw == 32 ? held_q<2, 1>(t.tz, nsm) : held_q<2, 2>(t.tz, nsm); break;
+    case 3: held = t.rw == 32 ? held_q<3, 1>(t.tz, nsm) : held_q<3, 2>(t.tz, nsm); break;
+    case 4: held = t.rw == 32 ? held_q<4, 1>(t.tz, nsm) : held_q<4, 2>(t.tz, nsm); break;
+    }
+    return ctas <= held;
 }
 
 size_t resident_inbox_bytes(int nz, int nx, int nbatch, int ns, const ResidentTile &t)
