@@ -453,7 +453,20 @@ def large_workload(nt=None, nshot=None):
                                       nrec=c["nrec"], snap_dt=c["snap_dt"], n_layers=8,
                                       vp_range=(1500.0, 4500.0), seed=77, surf_offset=0)
     sv.imaging_sign = 1
-    return sv, true, init
+    # In the cropped time the wave meets none of the cells where the two models
+    # part: three per cent throughout give the direct waves a residual.
+    return sv, true, tuple(0.97 * a for a in init)
+
+
+def compare_gradients(a, b):
+    """(equal bit for bit, largest relative L2 difference) of two runs' (L2,
+    gradients), which must be finite and not all zero: anything else compares
+    nothing."""
+    for L2, g in (a, b):
+        if not (np.isfinite(L2) and L2 > 0 and all(np.isfinite(x).all() and np.any(x) for x in g)):
+            raise RuntimeError("gradients to compare are not finite or all zero")
+    equal = a[0] == b[0] and all(np.array_equal(x, y) for x, y in zip(a[1], b[1]))
+    return bool(equal), max(float(np.linalg.norm(y - x) / np.linalg.norm(x)) for x, y in zip(a[1], b[1]))
 
 
 STEP_BYTES = {  # algorithmic bytes per grid-point update of a whole time step (FP32)
@@ -570,9 +583,7 @@ def c3_cropped(args, nt=240):
             out[storage] = dict(L2=L2, g=g, s=sec, kind=kind, seg=seg, slots=slots,
                                 gb=p.device_bytes / 1e9, shape=p.shape)
     f, k = out["full"], out["checkpoint"]
-    equal = f["L2"] == k["L2"] and all(np.array_equal(a, b) for a, b in zip(f["g"], k["g"]))
-    diff = max(float(np.linalg.norm(b - a) / max(np.linalg.norm(a), 1e-300))
-               for a, b in zip(f["g"], k["g"]))
+    equal, diff = compare_gradients((f["L2"], f["g"]), (k["L2"], k["g"]))
     upd = 2.0 * c["nshot"] * nt * c["nz"] * c["nx"]
     return {"workload": f"1001x2001, order 8, 64 shots, nt={nt} (cropped from 10000), FP32",
             "full_s": f["s"], "checkpoint_s": k["s"],
@@ -580,7 +591,7 @@ def c3_cropped(args, nt=240):
             "checkpoint_segment_steps": k["seg"], "checkpoint_slots_per_shot": k["slots"],
             "device_gb": {"full": f["gb"], "checkpoint": k["gb"]},
             "kernels": dict(zip(("family", "rows_per_thread", "block_y"), f["shape"])),
-            "checkpointed_equals_full_bitwise": bool(equal), "max_rel_l2_difference": diff}
+            "checkpointed_equals_full_bitwise": equal, "max_rel_l2_difference": diff}
 
 
 UNEVEN_SHOTS = 32
@@ -660,6 +671,8 @@ def forward_modes(plans, updates, rpt=0, by=4):
     t0 = time.perf_counter()
     engine.multi_forward(plans)
     conc = time.perf_counter() - t0
+    for p in plans:
+        p.forward()
     t0 = time.perf_counter()
     for p in plans:
         p.forward()
@@ -713,7 +726,8 @@ def small_surveys(args):
         each = [plan(2, 200 + k) for k in range(8)]
         one16 = plan(16, 300)
         engine.multi_gradient(each)  # tunes and captures graphs
-        one16.gradient(fetch=False)
+        for p in [*each, one16]:     # ... of each plan alone
+            p.gradient(fetch=False)
         t0 = time.perf_counter()
         engine.multi_gradient(each)
         conc = time.perf_counter() - t0

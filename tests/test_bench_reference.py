@@ -6,6 +6,8 @@ import os
 import subprocess
 import sys
 
+import pytest
+
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
@@ -116,3 +118,29 @@ def test_uneven_batch_configuration():
                                                 dptr(rho), dptr(lam), dptr(mu), dptr(sv.hc),
                                                 dptr(out))
         assert rc == _lib.PSV_OK and sv.dt < out[0], (k, out)
+
+
+def test_the_cropped_large_survey_has_a_residual_where_its_wave_gets():
+    # 240 steps at 4500 m/s cross some 54 cells: the models differ around every
+    # source, or the residual is exactly zero and the gradients are 0 / 0
+    import numpy as np
+    b = _bench_module()
+    sv, true, init = b.large_workload(nt=240, nshot=8)
+    for a, c in zip(true, init):
+        for z, x in zip(sv.z_src, sv.x_src):
+            assert np.all(a[z - 2:z + 20, x - 20:x + 21] != c[z - 2:z + 20, x - 20:x + 21])
+
+
+def test_gradients_that_compare_nothing_are_refused():
+    import numpy as np
+    b = _bench_module()
+    g = [np.arange(4.0) + k for k in range(3)]
+    assert b.compare_gradients((1.0, g), (1.0, [x.copy() for x in g])) == (True, 0.0)
+    equal, diff = b.compare_gradients((1.0, g), (1.0, [x * (1 + 1e-7) for x in g]))
+    assert not equal and 0 < diff < 1e-6
+    for bad in ([g[0], g[1] * np.nan, g[2]], [g[0], 0 * g[1], g[2]]):
+        for pair in (((1.0, bad), (1.0, g)), ((1.0, g), (1.0, bad))):
+            with pytest.raises(RuntimeError):
+                b.compare_gradients(*pair)
+    with pytest.raises(RuntimeError):
+        b.compare_gradients((0.0, g), (0.0, g))
