@@ -522,6 +522,49 @@ public:
     int par(int k) const { return fused() ? (k & 1) : 0; }
     static int v4_rpt(int r) { return (r == 1 || r == 2 || r == 4) ? r : 1; }
 
+    // Largest sum in a tile of tw x tz cells of the sources of a shot, a weight each,
+    // and the receivers.
+    int crowd(int tw, int tz, int source, int receiver) const
+    {
+        const int ntx = (sv.g.nx + tw - 1) / tw, ntz = (sv.g.nz + tz - 1) / tz;
+        std::vector<int> n((size_t)ntx * ntz, 0);
+        std::map<std::pair<int, int>, int> shot;  // sources by tile and shot
+        int most = 0;
+        for (int i = 0; receiver && i < sv.s.nrec; i++)
+            most = std::max(most, n[(size_t)(sv.z_rec[i] / tz) * ntx + sv.x_rec[i] / tw] += receiver);
+        for (int i = 0; i < sv.s.nsrc; i++) {
+            if (sv.fire[i] < 0 || sv.fire[i] >= sv.s.nshot) continue;
+            const int t = sv.z_src[i] / tz * ntx + sv.x_src[i] / tw;
+            most = std::max(most, (shot[{t, sv.fire[i]}] += source) + n[(size_t)t]);
+        }
+        return most;
+    }
+    // Whether sources or receivers crowd in tiles so that the direct kernels are
+    // faster.  One warp has a tile's sources to itself, which sum in their order, and
+    // one its receivers (in the list it is the same): 33 ns a source and 13 a receiver
+    // on chip, 35 and 20 in the list.  That against a gain of 4 to 5 us on chip, and
+    // of 5 us a million points by the list; with 100 receivers in every tile of the
+    // list half of that is left (direct / these kernels, modelling, order 4):
+    //   most sources of a shot in a tile
+    //     on chip, 101 x 201, 1 shot       1 2.33    64 2.19   128 1.14   176 0.85
+    //     on chip, 301 x 601, 1 shot       1 2.42    64 1.81   256 0.82
+    //     on chip, 281 x 561, 2 shots      1 1.85    64 1.49   256 0.80
+    //     list, 301 x 601, 8 shots         1 1.46   192 1.11   240 0.97   320 0.87
+    //     list, 1001 x 2001, 1 shot        1 1.51   192 1.22   264 1.01   384 0.90
+    //   most receivers in a tile
+    //     list, 301 x 601, 8 shots        64 1.45   128 1.42   512 1.04   896 0.71
+    //     list, 1001 x 2001, 1 shot       64 1.52   128 1.50   512 1.20   592 1.01   1008 0.73
+    //   receivers in every tile
+    //     on chip, 301 x 601, 1 shot      34 2.35   135 1.50   304 1.24   1216 0.52
+    //     on chip, 281 x 561, 2 shots     64 1.73   256 1.22   576 0.98   2304 0.35
+    //     list, 301 x 601, 8 shots        27 1.24   105 1.13   230 0.91   920 0.42
+    //     list, 1001 x 2001, 1 shot       27 1.04   105 1.03   230 0.84   920 0.41
+    bool chip_crowded() const { return rt.tz && 6.5e-3 * crowd(rt.rw, rt.tz, 5, 2) > 4.5; }
+    bool list_crowded() const
+    {
+        return 5e-3 * crowd(64, 16, 7, 4) > 5e-6 * sv.g.nz * sv.g.nx * B ||
+               sv.s.nrec > 150ll * ((sv.g.nx + 63) / 64) * ((sv.g.nz + 15) / 16);
+    }
     // Whether the plan may choose its kernels.
     bool any_kernels() const { return opt.kernel_family == 0 && opt.rows_per_thread == 0; }
     // The shape of a plan nobody autotunes (modelling).  A block shape or a chain
@@ -538,11 +581,12 @@ public:
     //   5          0.83 - 1.03   0.95 - 1.2  1.1 - 1.3   1.25 - 1.3   1.2 - 1.5
     //   7          0.92 - 1.2    1.03 - 1.3  1.2 - 1.4   1.2 - 1.3
     //   9 and 13   0.96 - 1.3    1.1 - 1.4   1.2 - 1.5   1.2 - 1.6
-    // (1001 x 2001, order 8, one shot: 40 against 21 us a step).
+    // (1001 x 2001, order 8, one shot: 40 against 21 us a step).  Neither where
+    // points crowd.
     int start_shape(int *r) const
     {
         const bool given = (opt.block_y > 0 && (opt.block_x <= 0 || opt.block_x == 32)) || opt.chains != 0;
-        if (rt.tz && !beside && !given) {
+        if (rt.tz && !beside && !given && !chip_crowded()) {
             *r = 8;
             return PSV_KERNELS_TMA;
         }
@@ -550,7 +594,7 @@ public:
         const double points = (double)sv.g.nz * sv.g.nx * B;
         const double least = bands >= 9 ? 0.5e6 : bands >= 5 ? 1e6 : 4e6;
         if (sizeof(T) == 4 && !given && bands >= 3 && points >= least &&
-            loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1)) {
+            loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) && !list_crowded()) {
             *r = 4;
             return PSV_KERNELS_TMA;
         }
@@ -1771,10 +1815,10 @@ public:
 
     int autotune(int nsteps, int *out_fam, int *out_rpt, int *out_by) override
     {
-        // (plans the loops cannot serve choose among other kernels)
+        // (plans the loops cannot serve, or not well, choose among other kernels)
         const TuneKey key{sv.g.nz, sv.g.nx, sv.ns, B, (int)sizeof(T),
                           opt.kernel_family + (loop_supported(16, sv.st, sv.sb, sv.sl, sv.sr, sv.nz1) ? 0 : 16) +
-                              (rt.tz && !beside ? 32 : 0)};
+                              (rt.tz && !beside ? 32 : 0) + (chip_crowded() ? 64 : 0) + (list_crowded() ? 128 : 0)};
         auto report = [&] {
             if (out_fam) *out_fam = fam;
             if (out_rpt) *out_rpt = rpt;
