@@ -489,8 +489,8 @@ def large_grid(args):
     - the headline roofline object: the dominant kernel's per-kernel
       algorithmic bytes (algorithmic_bytes x points) / its CUDA-event launch
       time, against the measured HBM copy bandwidth, with the ncu DRAM
-      traffic per launch (profiles/dram_traffic_large.txt, captured on two
-      shots and scaled to eight by the points processed);
+      traffic per launch (profiles/dram_traffic_large.txt, captured on eight
+      shots); of kernels that run many steps in a launch, all of a step;
     - the forward and adjoint time steps' fractions on the whole-step bytes
       (60 and 84 B per update), and with the We / snapshot-store and imaging
       terms added;

@@ -39,15 +39,16 @@
 // its next visitor through the same release / acquire chain; these are read
 // past L1 (ld.global.cg).
 //
-// What bounds it: on grids beyond L2, DRAM (1001 x 2001, order 8, three shots:
-// 51 B a point and step cross it against 76 for two launches) and the
-// shared-memory pipe, 55 % and 62 % busy; below, the latency from claim to
-// publication, about 4 us, against the items a half-step has.  us a step,
-// forward / adjoint, two launches before -> loop (TZ = 16):
-//   1001 x 2001 x 8, order 8   251 / 310 -> 210 / 280
+// What bounds it: on grids beyond L2, DRAM and the shared-memory pipe (1001 x
+// 2001, order 8, eight shots: 48 B a point and step cross DRAM in modelling, 66
+// in storing passes, 104 in the adjoint, against 61, 76 and 99 for two launches;
+// DRAM 55, 63 and 75 % busy, the pipe 58, 50 and 38 %); below, the latency from
+// claim to publication against the items a half-step has.  us a step, forward /
+// adjoint, two launches before -> loop (TZ = 16):
+//   1001 x 2001 x 8, order 8   251 / 310 -> 214 / 284
 //   1001 x 2001 x 3, order 8   modelling 145 (direct) -> 64
 //   601 x 1203 x 4, order 8    61 / 68 (direct, two chains) -> 36 / 50
-//   301 x 601 x 8, order 4     23.3 / 24.4 (direct, two chains) -> 18.2 / 24.0
+//   301 x 601 x 8, order 4     23.3 / 24.4 (direct, two chains) -> 17.8 / 22.5
 // Tried and slower: one row of warps per stage doing the keeper's work; two
 // rows per thread (20 % less shared-memory traffic, 3 x the time of a tile:
 // longer code run by fewer warps); two teams a CTA; four CTAs per SM at 64
@@ -124,7 +125,8 @@ struct Rec {
 };
 static_assert(sizeof(Rec) == 80, "record size");
 
-// n / d and n % d for 0 <= n < 2^31 by multiplication.
+// n / d and n % d for 0 <= n < 2^31 by multiplication (Granlund and Montgomery,
+// Division by invariant integers using multiplication, 1994).
 struct FastDiv {
     unsigned m, s, d;
     __device__ void set(unsigned div)

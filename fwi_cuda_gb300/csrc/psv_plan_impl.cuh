@@ -503,7 +503,12 @@ public:
     {
         if constexpr (sizeof(T) == 4) {
             const int most = loop_max_steps(sv.g.nz, sv.g.nx, B);
-            // the fields a step touches, against what L2 holds beside the rest
+            // The fields a step touches, against what L2 holds beside the rest: far
+            // items are prefetched when claimed.  us a step near / far: storing forward,
+            // order 8, 35 MB 18.3 / 19.0, 70 MB 36.0 / 35.7, 88 MB 47.8 / 46.7, 140 MB
+            // 80.4 / 74.8, 390 MB 231 / 214; order 4 the same ratios; adjoint, order 4,
+            // 47 MB 22.0 / 22.7, 94 MB 47.3 / 47.3, 141 MB 75.9 / 73.6; order 8, 94 MB
+            // 49.7 / 52.5, 187 MB 102.4 / 103.3, 520 MB 289 / 284.
             const double state = (mode == MODE_ADJ ? 8.0 : mode == MODE_FWD ? 6.0 : 5.0) * plane * B * sizeof(T);
             const int far = state > 90e6;
             for (int j = 0; j < n; j += most) {

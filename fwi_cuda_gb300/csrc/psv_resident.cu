@@ -23,8 +23,10 @@
 //   301 x 601, 1 shot, order 4    3.6 / 4.0   (32 x 38)
 //   281 x 561, 2 shots, order 4   6.9 / 8.0   (64 x 36; 13.1 / 14.6 by psv_loop.cu)
 // and whole passes, two launches a step before -> here: 400 steps of modelling
-// on the first grid 3676 -> 1377 us, the second's gradient (800 steps)
-// 9292 -> 4680, five shots on 187 x 133, order 6, 1000 steps 10595 -> 4627.
+// on the first grid 3591 -> 1322 us, the second's gradient (800 steps)
+// 9264 -> 3992, five shots on 187 x 133, order 6, 1000 steps 10478 -> 4618.
+// At 128 registers a thread (512 threads may fill an SM) every instantiation
+// spills: 144 to 296 bytes stored with one quad a thread, 8 to 168 with two.
 // What neither the next update nor a neighbour waits for comes after the rim
 // of v is sent: snapshots, imaging, traces; source amplitudes are fetched
 // before the waits.  The traces' FP64 divide, at a 64th of the FP32 rate, held

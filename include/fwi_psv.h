@@ -156,8 +156,9 @@ typedef struct psv_options {
                                    1, 2, 4; FUSED family: tile rows 16 or 32; MARCH family:
                                    rows each CTA marches, 32, 64 or 128; 0 = default */
     int kernel_family;          /* time-step kernels: 0 = any (the autotuner chooses; before
-                                   and without it, by the batch's grid points, or the direct
-                                   family where block_y (block_x 0 or 32) or chains is given),
+                                   and without it, by the batch's grid points and how its
+                                   sources and receivers crowd, or the direct family where
+                                   block_y (block_x 0 or 32) or chains is given),
                                    PSV_KERNELS_DIRECT, _TMA, _VEC4, _FUSED or _MARCH (the
                                    last four FP32 only; FUSED needs no free surface but a top
                                    one, MARCH none or a top one on the first interior row) */
@@ -467,7 +468,10 @@ long long psv_plan_kernel_launches(const psv_plan *plan);
  * nsteps adjoint steps of the first batch, each kernel bracketed by CUDA
  * events on the plan's stream.  ms6 = mean milliseconds per launch of
  * {stress, velocity, 0} forward, then the same adjoint (sources and
- * receivers run inside the velocity kernel; slots 2 and 5 stay 0).
+ * receivers run inside the velocity kernel; slots 2 and 5 stay 0).  Kernels
+ * that run whole steps have no launch of a half-step: the stress slot is 0 and
+ * the velocity slot the mean of a step (FUSED and MARCH: of a launch; TMA with
+ * many steps a launch: the pass's time over its steps).
  * Needs a model and observed traces; leaves the wavefields undefined. */
 int psv_profile_kernels(psv_plan *plan, int nsteps, double *ms6);
 
