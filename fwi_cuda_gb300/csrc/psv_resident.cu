@@ -26,7 +26,7 @@
 // on the first grid 3591 -> 1322 us, the second's gradient (800 steps)
 // 9264 -> 3992, five shots on 187 x 133, order 6, 1000 steps 10478 -> 4618.
 // At 128 registers a thread (512 threads may fill an SM) every instantiation
-// spills: 144 to 296 bytes stored with one quad a thread, 8 to 168 with two.
+// spills: 180 to 296 bytes stored with one quad a thread, 16 to 168 with two.
 // What neither the next update nor a neighbour waits for comes after the rim
 // of v is sent: snapshots, imaging, traces; source amplitudes are fetched
 // before the waits.  The traces' FP64 divide, at a 64th of the FP32 rate, held
